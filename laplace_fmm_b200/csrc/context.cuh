@@ -42,6 +42,9 @@ struct DevTables {
 	// Wigner small-d matrices (N = 18 layout) for each theta slot
 	double* dmat = nullptr;
 	int n_dslots = 0;
+	// the same matrices as FP64 MMA fragments of the real (.x) and imaginary
+	// (.y) parts' blocks (rot.cuh), [slot][fragment][32 lanes]
+	double2* rotf = nullptr;
 	// (cos m phi, sin m phi), m < 18, for each phi slot
 	double2* emat = nullptr;
 	int n_eslots = 0;

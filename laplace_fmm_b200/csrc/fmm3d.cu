@@ -8,6 +8,7 @@
 // no atomics and no per-thread local arrays.
 #include "fmm3d.cuh"
 #include "m2l_gemm.cuh"
+#include "rot.cuh"
 #include <algorithm>
 
 namespace lfmm {
@@ -499,30 +500,55 @@ int fmm3d_solve_device(Context& ctx, const ParticleInput& in, int N, int depth, 
 	size_t lo = depth > 2 ? t.loff[2] : t.ncells;
 	LFMM_CUDA(ctx, cudaMemsetAsync(E.inner, 0, sizeof(double2) * lo * E.Nx2, s));
 	// upward
-	p2m_kernel<<<div_up(t.lsize[LL], WPB), WPB * 32, 0, s>>>(t, E, ctx.tables.d.knm);
-	for (int L = depth - 2; L >= 0; --L)
-		m2m_kernel<<<div_up(t.lsize[L], WPB), WPB * 32, 0, s>>>(t, E, L, ctx.tables.d, ctx.dev_flags);
+	if (depth > 2)                         // no far pairs on levels 0 and 1
+		p2m_kernel<<<div_up(t.lsize[LL], WPB), WPB * 32, 0, s>>>(t, E, ctx.tables.d.knm);
+	// factored translations unless the per-pair rotations are asked for; the
+	// upward pass ends at level 2, the coarsest with far pairs
+	const bool rot = ctx.m2l_engine != 1;
+	const double* ax = nullptr;
+	if (rot && depth > 2) {
+		double h[MAX_LEVELS];
+		for (int L = 0; L < depth; ++L) h[L] = t.geo_host[3] / (double)(1ull << L);
+		if (!(ax = rot_axial_tables(ctx, N, h, depth, false))) return ERR_OOM;
+	}
+	auto flat = [&](double2* e, int L) { return reinterpret_cast<double*>(e + t.loff[L] * E.Nx2); };
+	for (int L = depth - 2; L >= 2; --L) {
+		if (rot) {
+			M2LPlan mp;
+			if ((st = m2m_plan_build(ctx, t, L, mp))) return st;
+			if ((st = rot_translate<double>(ctx, ROT_M2M, mp, flat(E.outer, L + 1), flat(E.outer, L), N,
+			                                rot_axial_level(ax, N, L))))
+				return st;
+		} else {
+			m2m_kernel<<<div_up(t.lsize[L], WPB), WPB * 32, 0, s>>>(t, E, L, ctx.tables.d, ctx.dev_flags);
+		}
+	}
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[2], s));
 	// downward
-	const bool gemm = ctx.m2l_engine != 1 && m2l_gemm_supported(N);     // FP64: SIMT GEMMs unless rotations asked
+	std::vector<M2LPlan> plans(depth);
 	for (int L = 2; L < depth; ++L) {
-		if (gemm) {
-			double h = t.geo_host[3] / (double)(1ull << L);
-			double* ops = m2l_ops_fp64(ctx, N, h);
-			if (!ops) return ERR_OOM;
-			M2LPlan plan;
-			if ((st = m2l_plan_build(ctx, t, L, plan))) return st;
-			const size_t off = t.loff[L] * E.Nx2;
-			if ((st = m2l_gemm<double>(ctx, plan, ops, reinterpret_cast<const double*>(E.outer + off),
-			                           reinterpret_cast<double*>(E.inner + off), N)))
+		if (rot) {
+			if ((st = m2l_plan_build(ctx, t, L, plans[L]))) return st;
+			if ((st = rot_translate<double>(ctx, ROT_M2L, plans[L], flat(E.outer, L), flat(E.inner, L), N,
+			                                rot_axial_level(ax, N, L))))
 				return st;
 		} else {
 			m2l_kernel<<<div_up(t.lsize[L], WPB), WPB * 32, 0, s>>>(t, E, L, ctx.tables.d, ctx.dev_flags);
 		}
 	}
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[3], s));
-	for (int L = 3; L < depth; ++L)
-		l2l_kernel<<<div_up(t.lsize[L], WPB), WPB * 32, 0, s>>>(t, E, L, ctx.tables.d, ctx.dev_flags);
+	for (int L = 3; L < depth; ++L) {
+		if (rot) {
+			// the level's cells grouped by octant (its M2L plan), one slot: the parent
+			M2LPlan lp = plans[L];
+			lp.vtab = t.parent + t.loff[L];
+			if ((st = rot_translate<double>(ctx, ROT_L2L, lp, flat(E.inner, L - 1), flat(E.inner, L), N,
+			                                rot_axial_level(ax, N, L))))
+				return st;
+		} else {
+			l2l_kernel<<<div_up(t.lsize[L], WPB), WPB * 32, 0, s>>>(t, E, L, ctx.tables.d, ctx.dev_flags);
+		}
+	}
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[4], s));
 	leaves_kernel<<<(unsigned)t.lsize[LL], LEAF_THREADS, 0, s>>>(t, E, ctx.tables.d.knm, pot, field);
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[5], s));

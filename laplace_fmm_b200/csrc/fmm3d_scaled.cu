@@ -1,11 +1,12 @@
 // 3D FMM in scaled expansions on the adaptive-form tree (uniform when
 // max_leaf = 0): plain FP64 or mixed (FP32 expansions and near field, FP64
 // M2L accumulation on levels 2-3, FP64 tile sums and self term).
-// Passes: P2M (every leaf, any level) -> M2M -> M2L (V, direction GEMMs) ->
+// Passes: P2M (every leaf, any level) -> M2M -> M2L (V) ->
 // P2L (X) -> L2L -> leaves: P2P (self + U), M2P (W), L2P.
 #include <cmath>
 #include "scaled_kernels.cuh"
 #include "m2l_tc.cuh"
+#include "rot.cuh"
 #include <algorithm>
 
 namespace lfmm {
@@ -52,17 +53,11 @@ template <typename real> Tab<real> tables_of(const DevTables& T);
 template <> Tab<double> tables_of<double>(const DevTables& T) { return Tab<double>{T.dmat, T.emat, T.m2m, T.l2l, T.knm, T.dirinfo}; }
 template <> Tab<float> tables_of<float>(const DevTables& T) { return Tab<float>{T.dmat_f, T.emat_f, T.m2m_f, T.l2l_f, T.knm_f, T.dirinfo}; }
 
-template <typename real> const real* ops_of(Context& ctx, int N);
-template <> const double* ops_of<double>(Context& ctx, int N) { return m2l_ops_fp64(ctx, N, 1.0); }
-template <> const float* ops_of<float>(Context& ctx, int N) { return m2l_ops_fp32(ctx, N); }
-
-// Dense FP64 scaled M2M (OP = SOP_M2M) or L2L operators, one per child octant
-// o (the octant bits of the child's code): column r is translate_scaled, the
-// rotation-based shift of the SIMT kernels, applied to the r-th unit vector.
-// out: [8][MT][MT], pre-zeroed.
-template <int OP>
-__global__ void __launch_bounds__(WPB * 32) shift_ops_kernel(int N, int MT, Tab<double> T, double* __restrict__ out,
-                                                             unsigned* flags)
+// Dense FP64 scaled M2M operators, one per child octant o (the octant bits
+// of the child's code): column r is translate_scaled applied to the r-th unit
+// vector.  out: [8][MT][MT], pre-zeroed.
+__global__ void __launch_bounds__(WPB * 32) m2m_ops_kernel(int N, int MT, Tab<double> T, double* __restrict__ out,
+                                                           unsigned* flags)
 {
 	__shared__ SmemT<double> sm[WPB];
 	__shared__ double2 unit[WPB][NX2MAX];
@@ -72,14 +67,14 @@ __global__ void __launch_bounds__(WPB * 32) shift_ops_kernel(int N, int MT, Tab<
 	const int o = (int)(task / R), r = (int)(task % R);
 	if (o >= 8) return;
 	const int bx = (o >> 2) & 1, by = (o >> 1) & 1, bz = o & 1;
-	const int d = OP == SOP_M2M ? dir_id(2 * bx - 1, 2 * by - 1, 2 * bz - 1) : dir_id(1 - 2 * bx, 1 - 2 * by, 1 - 2 * bz);
+	const int d = dir_id(2 * bx - 1, 2 * by - 1, 2 * bz - 1);
 	for (int c = lane; c < Nx2; c += 32)
 		unit[w][c] = make_double2(c == r / 2 && !(r & 1) ? 1.0 : 0.0, c == r / 2 && (r & 1) ? 1.0 : 0.0);
 	__syncwarp();
 	double2 acc[CMAX];
 #pragma unroll
 	for (int k = 0; k < CMAX; ++k) acc[k] = make_double2(0.0, 0.0);
-	translate_scaled<OP, double>(unit[w], d, acc, N, Nx2, sm[w], T, flags);
+	translate_scaled(unit[w], d, acc, N, Nx2, sm[w], T, flags);
 	double* op = out + (size_t)o * MT * MT;
 #pragma unroll
 	for (int k = 0; k < CMAX; ++k) {
@@ -91,56 +86,37 @@ __global__ void __launch_bounds__(WPB * 32) shift_ops_kernel(int N, int MT, Tab<
 	}
 }
 
-// Moves the diagonal of the 8 FP64 operators [8][MT][MT] into diag [8][MT]
-// (FP32; zero past R) and zeroes it in the operators.
-__global__ void split_diag_kernel(double* __restrict__ ops64, int MT, int R, float* __restrict__ diag)
-{
-	const int e = blockIdx.x * blockDim.x + threadIdx.x;
-	if (e >= 8 * MT) return;
-	const int o = e / MT, c = e % MT;
-	double* p = ops64 + ((size_t)o * MT + c) * MT + c;
-	diag[e] = c < R ? (float)*p : 0.f;
-	*p = 0.0;
-}
-
-// The tensor-core M2M (op 0) or L2L (op 1, followed by its diagonal) operators
-// of order N, cached in the context (built once; the plan's warm solves build
-// them before capture).  nullptr on failure, with st = ERR_OOM or ERR_CUDA.
-const uint4* shift_ops_tc(Context& ctx, int N, int op, int& st)
+// The tensor-core M2M operators of order N, cached in the context (built
+// once; the plan's warm solves build them before capture).  nullptr on
+// failure, with st = ERR_OOM or ERR_CUDA.
+const uint4* m2m_ops_tc(Context& ctx, int N, int& st)
 {
 	st = OK;
-	const int tag = 30 + op;
+	constexpr int tag = 30;
 	for (auto& e : ctx.opcache)
 		if (e.N == N && e.prec == tag) { e.stamp = ++ctx.opcache_clock; return static_cast<const uint4*>(e.ptr); }
 	const int MT = m2l_padded(N), R = N * (N + 1);
 	const size_t bytes64 = sizeof(double) * 8 * (size_t)MT * MT;
-	const size_t bytes_tc = tc_ops_bytes(8, N) + (op == 1 ? sizeof(float) * 8 * MT : 0);
+	const size_t bytes_tc = tc_ops_bytes(8, N);
 	opcache_make_room(ctx);
 	double* d = nullptr;
 	void* tc = nullptr;
 	if (cudaMalloc(&d, bytes64) != cudaSuccess || cudaMalloc(&tc, bytes_tc) != cudaSuccess) {
 		cudaGetLastError();
 		if (d) cudaFree(d);
-		ctx.last_error = "shift operators: out of memory";
+		ctx.last_error = "M2M operators: out of memory";
 		st = ERR_OOM;
 		return nullptr;
 	}
-	const Tab<double> T = tables_of<double>(ctx.tables.d);
-	const size_t tasks = (size_t)8 * R;
 	cudaMemsetAsync(d, 0, bytes64, ctx.stream);
-	if (op == 0) {
-		shift_ops_kernel<SOP_M2M><<<div_up(tasks, WPB), WPB * 32, 0, ctx.stream>>>(N, MT, T, d, ctx.dev_flags);
-	} else {
-		shift_ops_kernel<SOP_L2L><<<div_up(tasks, WPB), WPB * 32, 0, ctx.stream>>>(N, MT, T, d, ctx.dev_flags);
-		split_diag_kernel<<<div_up(8 * MT, 256), 256, 0, ctx.stream>>>(
-			d, MT, R, reinterpret_cast<float*>(static_cast<uint8_t*>(tc) + tc_ops_bytes(8, N)));
-	}
+	m2m_ops_kernel<<<div_up((size_t)8 * R, WPB), WPB * 32, 0, ctx.stream>>>(N, MT, tables_of<double>(ctx.tables.d), d,
+	                                                                        ctx.dev_flags);
 	st = cudaGetLastError() == cudaSuccess ? tc_ops_convert(ctx, d, 8, N, tc) : ERR_CUDA;
 	if (cudaStreamSynchronize(ctx.stream) != cudaSuccess) st = ERR_CUDA;
 	cudaFree(d);
 	if (st != OK) {
 		cudaFree(tc);
-		ctx.last_error = "shift operators: build failed";
+		ctx.last_error = "M2M operators: build failed";
 		return nullptr;
 	}
 	OpCacheEntry e;
@@ -150,34 +126,16 @@ const uint4* shift_ops_tc(Context& ctx, int N, int op, int& st)
 	return static_cast<const uint4*>(tc);
 }
 
-// M2M plan of level L for the tensor-core engine: the non-leaf cells (order,
-// one class; a leaf keeps its P2M expansion) and their children by octant
-// (vtab[cell][8]: level-local index at L + 1, or -1).
-__global__ void m2m_plan_kernel(DevTree t, int L, int32_t* __restrict__ vtab, int32_t* __restrict__ order,
-                                uint32_t* __restrict__ count)
-{
-	const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (c >= t.lsize[L]) return;
-	const size_t g = t.loff[L] + c, cb = t.loff[L + 1];
-	if (t.beg[g] >= t.end[g]) return;
-	for (uint32_t k = t.beg[g]; k < t.end[g]; ++k) vtab[c * 8 + (size_t)(t.code[cb + k] & 7ull)] = (int32_t)k;
-	order[atomicAdd(count, 1u)] = (int32_t)c;
-}
-
-int m2m_plan_build(Context& ctx, const DevTree& t, int L, M2LPlan& plan)
-{
-	const size_t m = t.lsize[L];
-	plan.cells = m;
-	plan.vtab = static_cast<int32_t*>(ctx.arena.take(sizeof(int32_t) * 8 * m));
-	plan.order = static_cast<int32_t*>(ctx.arena.take(sizeof(int32_t) * m));
-	plan.oct_count = static_cast<uint32_t*>(ctx.arena.take(sizeof(uint32_t) * 8));
-	if (!plan.vtab || !plan.order || !plan.oct_count) { ctx.last_error = "m2m plan: allocation failed"; return ERR_OOM; }
-	LFMM_CUDA(ctx, cudaMemsetAsync(plan.vtab, 0xff, sizeof(int32_t) * 8 * m, ctx.stream));
-	LFMM_CUDA(ctx, cudaMemsetAsync(plan.oct_count, 0, sizeof(uint32_t) * 8, ctx.stream));
-	m2m_plan_kernel<<<div_up(m, 256), 256, 0, ctx.stream>>>(t, L, plan.vtab, plan.order, plan.oct_count);
-	LFMM_CUDA(ctx, cudaGetLastError());
-	return OK;
-}
+// Levels of the mixed form's FP32 expansions that take the factored FP64
+// translations instead of the tensor-core engine (B200, rot_kernel against
+// m2l_tc_kernel, us).  M2L: a tensor-core launch costs 105-240 (N = 8-18) on
+// the smallest levels, where its 128-target tiles are mostly empty; the
+// factored one 20-105 up to 150 cells, 46 / 94 / 187 / 256 (N = 8 / 12 / 16 /
+// 18) at 300-512 cells, 136 / 298 / 615 / 837 at 1341, against 142 / 172 / 240
+// / 306 for the tensor cores: the line lies at 512.  M2M at N = 16: 51 / 61 /
+// 87 / 90 at 55 / 1341 / 4169 / 4096 cells against 82-136, but 625 against
+// 281 at 32,768.
+constexpr size_t ROT_M2L_CELLS = 512, ROT_M2M_CELLS = 6144;
 
 template <typename real>
 int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, SolveStats* stats,
@@ -196,12 +154,8 @@ int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, S
 	real* qr = static_cast<real*>(ctx.arena.take(sizeof(real) * n));
 	v2* outer = static_cast<v2*>(ctx.arena.take(sizeof(v2) * C * Nx2));
 	v2* inner = static_cast<v2*>(ctx.arena.take(sizeof(v2) * C * Nx2));
-	size_t bmax = 0;
-	for (int L = 0; L < t.depth; ++L) bmax = std::max(bmax, t.lsize[L]);
 	const bool coarse64 = sizeof(real) == sizeof(float);
-	double* cv_in = coarse64 ? static_cast<double*>(ctx.arena.take(sizeof(double) * bmax * R)) : nullptr;
-	double* cv_out = coarse64 ? static_cast<double*>(ctx.arena.take(sizeof(double) * bmax * R)) : nullptr;
-	if (!xr || !yr || !zr || !qr || !outer || !inner || (coarse64 && (!cv_in || !cv_out))) {
+	if (!xr || !yr || !zr || !qr || !outer || !inner) {
 		ctx.last_error = "scaled solve: allocation failed";
 		return ERR_OOM;
 	}
@@ -212,47 +166,48 @@ int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, S
 	LFMM_CUDA(ctx, cudaMemsetAsync(inner, 0, sizeof(v2) * C * Nx2, s));
 	const unsigned nl = (unsigned)t.nleaves;
 	relcoords_kernel<real><<<nl, 128, 0, s>>>(t, xr, yr, zr, qr);
-	p2m_scaled_kernel<real><<<div_up(nl, WPB), WPB * 32, 0, s>>>(t, xr, yr, zr, qr, N, knm, outer);
+	if (t.depth > 2)                       // multipoles below level 2 reach nothing
+		p2m_scaled_kernel<real><<<div_up(nl, WPB), WPB * 32, 0, s>>>(t, xr, yr, zr, qr, N, knm, outer);
 	int st;
-	// the FP32 levels' shifts on the tensor-core engine (dense scaled operators,
-	// one per child octant), else the rotation-based SIMT kernels
-	const bool tc_shift = sizeof(real) == sizeof(float) && ctx.m2l_engine == 3 && m2l_tc_supported(N);
-	if (tc_shift) {
-		const uint4* mops = shift_ops_tc(ctx, N, 0, st);
-		if (!mops) return st;
-		for (int L = t.depth - 2; L >= 0; --L) {
-			if (t.lsize[L] == 0) continue;
-			M2LPlan mp;
-			if ((st = m2m_plan_build(ctx, t, L, mp))) return st;
-			if ((st = shift_gemm_tc(ctx, TC_M2M, mp, mops, reinterpret_cast<const float*>(outer + t.loff[L + 1] * Nx2),
-			                        reinterpret_cast<float*>(outer + t.loff[L] * Nx2), N, t.lsize[L + 1])))
-				return st;
+	// the tensor-core engine on the FP32 expansions' larger levels (M2L; M2M
+	// through dense scaled operators, one per child octant)
+	const bool tc = sizeof(real) == sizeof(float) && ctx.m2l_engine == 3 && m2l_tc_supported(N);
+	// every other translation (the FP64 form's, the mixed form's L2L, the M2L of
+	// its levels 2 and 3, its small levels) goes through the factored FP64
+	// engine; the upward pass ends at level 2, the coarsest whose multipoles
+	// anything reads
+	const double unit_h = 1.0;
+	const double* ax = t.depth > 2 ? rot_axial_tables(ctx, N, &unit_h, 1, true) : nullptr;
+	if (t.depth > 2 && !ax) return ERR_OOM;
+	auto flat = [&](v2* e, int L) { return reinterpret_cast<real*>(e + t.loff[L] * Nx2); };
+	for (int L = t.depth - 2; L >= 2; --L) {
+		if (t.lsize[L] == 0) continue;
+		M2LPlan mp;
+		if ((st = m2m_plan_build(ctx, t, L, mp))) return st;
+		if (tc && t.lsize[L] > ROT_M2M_CELLS) {
+			const uint4* mops = m2m_ops_tc(ctx, N, st);
+			if (!mops) return st;
+			st = m2m_gemm_tc(ctx, mp, mops, reinterpret_cast<const float*>(outer + t.loff[L + 1] * Nx2),
+			                 reinterpret_cast<float*>(outer + t.loff[L] * Nx2), N, t.lsize[L + 1]);
+		} else {
+			st = rot_translate<real>(ctx, ROT_M2M, mp, flat(outer, L + 1), flat(outer, L), N, ax);
 		}
-	} else {
-		for (int L = t.depth - 2; L >= 0; --L)
-			m2m_scaled_kernel<real><<<div_up(t.lsize[L], WPB), WPB * 32, 0, s>>>(t, L, outer + t.loff[L + 1] * Nx2,
-			                                                                     outer + t.loff[L] * Nx2, N, T,
-			                                                                     ctx.dev_flags);
+		if (st) return st;
 	}
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[2], s));
 	std::vector<M2LPlan> plans(t.depth);
 	if (t.depth > 2) {
-		const real* ops = ops_of<real>(ctx, N);
-		const double* opd = coarse64 ? m2l_ops_fp64(ctx, N, 1.0) : nullptr;
-		if (!ops || (coarse64 && !opd)) return ERR_OOM;
 		for (int L = 2; L < t.depth; ++L) {
 			if (t.lsize[L] == 0) continue;
 			M2LPlan& plan = plans[L];
 			if ((st = m2l_plan_build(ctx, t, L, plan))) return st;
 			const real* mL = reinterpret_cast<const real*>(outer + t.loff[L] * Nx2);
 			real* lL = reinterpret_cast<real*>(inner + t.loff[L] * Nx2);
-			if (coarse64 && L <= 3) {
-				// FP64 accumulation on the coarse levels
-				size_t m = t.lsize[L] * (size_t)R;
-				convert_kernel<real><<<div_up(m, 256), 256, 0, s>>>(mL, cv_in, m);
-				if ((st = m2l_gemm<double>(ctx, plan, opd, cv_in, cv_out, N))) return st;
-				convert_back_kernel<real><<<div_up(m, 256), 256, 0, s>>>(cv_out, lL, m);
-			} else if (sizeof(real) == sizeof(float) && ctx.m2l_engine == 3 && m2l_tc_supported(N)) {
+			// a level's own source order (level_N) is the tensor-core engine's
+			const bool own_n = level_N && level_N[L] > 0 && level_N[L] < N;
+			if (!coarse64 || L <= 3 || (tc && t.lsize[L] <= ROT_M2L_CELLS && !own_n)) {
+				if ((st = rot_translate<real>(ctx, ROT_M2L, plan, mL, lL, N, ax))) return st;
+			} else if (tc) {
 				// tcgen05 hi/lo GEMM on the FP32 levels (FP16 or TF32 operands)
 				float t_inv = 1.f;
 				const uint4* tc = m2l_ops_tc(ctx, N, &t_inv);
@@ -261,31 +216,23 @@ int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, S
 				                      level_N ? level_N[L] : 0, t_inv)))
 					return st;
 			} else {
-				if ((st = m2l_gemm<real>(ctx, plan, ops, mL, lL, N))) return st;
+				const float* ops = m2l_ops_fp32(ctx, N);
+				if (!ops) return ERR_OOM;
+				if ((st = m2l_gemm(ctx, plan, ops, reinterpret_cast<const float*>(mL), reinterpret_cast<float*>(lL), N)))
+					return st;
 			}
 		}
 	}
 	if (t.adaptive && t.n_x > 0)
 		p2l_kernel<real><<<div_up(C, WPB), WPB * 32, 0, s>>>(t, N, knm, inner);
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[3], s));
-	if (tc_shift && t.depth > 3) {
-		const uint4* lops = shift_ops_tc(ctx, N, 1, st);
-		if (!lops) return st;
-		for (int L = 3; L < t.depth; ++L) {
-			if (t.lsize[L] == 0) continue;
-			// the level's cells grouped by octant (its M2L plan), one slot: the parent
-			M2LPlan lp = plans[L];
-			lp.vtab = t.parent + t.loff[L];
-			if ((st = shift_gemm_tc(ctx, TC_L2L, lp, lops, reinterpret_cast<const float*>(inner + t.loff[L - 1] * Nx2),
-			                        reinterpret_cast<float*>(inner + t.loff[L] * Nx2), N, t.lsize[L - 1])))
-				return st;
-		}
-	} else {
-		for (int L = 3; L < t.depth; ++L)
-			if (t.lsize[L])
-				l2l_scaled_kernel<real><<<div_up(t.lsize[L], WPB), WPB * 32, 0, s>>>(t, L, inner + t.loff[L - 1] * Nx2,
-				                                                                     inner + t.loff[L] * Nx2, N, T,
-				                                                                     ctx.dev_flags);
+	for (int L = 3; L < t.depth; ++L) {
+		if (t.lsize[L] == 0) continue;
+		// the level's cells grouped by octant (its M2L plan), one slot: the parent
+		M2LPlan lp = plans[L];
+		lp.vtab = t.parent + t.loff[L];
+		st = rot_translate<real>(ctx, ROT_L2L, lp, flat(inner, L - 1), flat(inner, L), N, ax);
+		if (st) return st;
 	}
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[4], s));
 	if constexpr (sizeof(real) == sizeof(float)) {

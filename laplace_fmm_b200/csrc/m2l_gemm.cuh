@@ -40,9 +40,8 @@ inline bool m2l_gemm_supported(int N) { return m2l_padded(N) <= 352; }
 int m2l_plan_build(Context& ctx, const DevTree& t, int L, M2LPlan& plan);
 
 // loc[c] = sum_slots T[dir] mult[src]   for every cell c of the level
-// (real = double: plain form; float: mixed form).  ops: [343][MT][MT].
-template <typename real>
-int m2l_gemm(Context& ctx, const M2LPlan& plan, const real* ops, const real* mult, real* loc, int N);
+// (FP32, partial sums carried in FP64).  ops: [343][MT][MT].
+int m2l_gemm(Context& ctx, const M2LPlan& plan, const float* ops, const float* mult, float* loc, int N);
 
 // 2D (FP64, expansions [cell][N] complex): the quadrant classes' 27 far
 // slots, the dense operators [49][MT][MT] (MT = 2N rounded up to 16) of cell

@@ -314,11 +314,7 @@ __device__ __forceinline__ int dir_d2(int dir)
 // previous item has completed by then).
 // MODE picks the operator of a (class, slot) and the store:
 //   TC_M2L    189 far slots, operator c_tc_slot_dir[class][slot], loc = sum;
-//   TC_M2M    8 slots (child octants), operator = slot, loc = sum;
-//   TC_L2L    1 slot (the parent), operator = class (the child's octant)
-//             without its diagonal, loc += sum + diag[class] * parent (the
-//             diagonal, 2^-(n+1) on degree n, applied exactly in FP32: through
-//             the TF32 split the dominant coefficients would lose 2^-22 per level).
+//   TC_M2M    8 slots (child octants), operator = slot, loc = sum.
 // The K blocks of a slot are fed from the highest degrees down, so the
 // dominant low-degree products enter each FP32 accumulator last, when the
 // accumulator's own rounding has least left to act on.
@@ -373,14 +369,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 m2l_tc_kernel(const uint8_t* __restrict__ ops, const float* __restrict__ mult, float* __restrict__ loc,
               const int32_t* __restrict__ vtab, const int32_t* __restrict__ order,
               const uint32_t* __restrict__ oct_count, int R, float* __restrict__ part, size_t cells,
-              const float* __restrict__ diag, unsigned* flags, const TcTrunc trunc, size_t src_cells, int ndir,
+              unsigned* flags, const TcTrunc trunc, size_t src_cells, int ndir,
               unsigned* __restrict__ work, int S, unsigned total, const unsigned* __restrict__ bmax, float t_inv,
               const uint4* __restrict__ shi, const uint4* __restrict__ slo,
               const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CUtensorMap tm_lo, int zero_row)
 {
 	static_assert(!F16 || MODE == TC_M2L, "FP16 operands: M2L only");
 	static_assert(!TMA || F16, "TMA row gathers: FP16 staged sources only");
-	using C = TcCfg<NC, NA, MODE != TC_L2L && !TMA, F16>;
+	using C = TcCfg<NC, NA, !TMA, F16>;
 	constexpr int UPB = C::UPB;
 	extern __shared__ uint8_t dsm[];
 	constexpr int NSTAGE = C::NSTAGE;
@@ -598,7 +594,7 @@ m2l_tc_kernel(const uint8_t* __restrict__ ops, const float* __restrict__ mult, f
 			if (nact > 0) gather(0, (active_kb[0] - 1) * UPB, nxt);
 			for (int j = 0; j < nact; ++j) {
 				const int slot = active[j];
-				int dir = MODE == TC_M2L ? c_tc_slot_dir[oct][slot] : MODE == TC_M2M ? slot : oct;
+				int dir = MODE == TC_M2L ? c_tc_slot_dir[oct][slot] : slot;
 				if (dir < 0 || dir >= ndir) {                   // an operator outside the set: reported
 					if (tid == 0) atomicOr(flags, DEV_ERR_RANGE);
 					dir = 0;
@@ -789,18 +785,6 @@ m2l_tc_kernel(const uint8_t* __restrict__ ops, const float* __restrict__ mult, f
 				atomicOr(flags, DEV_ERR_RANGE);
 				store = false;
 			}
-			const float* xs = nullptr;
-			const float* dg = nullptr;
-			if (MODE == TC_L2L && store) {
-				const int par = vtab[tg];
-				if (par < 0 || (size_t)par >= src_cells) {
-					atomicOr(flags, DEV_ERR_RANGE);
-					store = false;
-				} else {
-					xs = mult + (size_t)par * R;
-					dg = diag + oct * NC;
-				}
-			}
 			if (store) {
 				const int c0 = half * W;
 				float* o = out + (size_t)tg * R + c0;
@@ -808,8 +792,7 @@ m2l_tc_kernel(const uint8_t* __restrict__ ops, const float* __restrict__ mult, f
 #pragma unroll
 				for (int c = 0; c < W; ++c)
 					if (c < lim) {
-						if (MODE == TC_L2L) o[c] += acc[c] + dg[c0 + c] * xs[c0 + c];
-						else if constexpr (F16) o[c] = acc[c] * out_scale;
+						if constexpr (F16) o[c] = acc[c] * out_scale;
 						else o[c] = acc[c];
 					}
 			}
@@ -831,8 +814,7 @@ m2l_tc_kernel(const uint8_t* __restrict__ ops, const float* __restrict__ mult, f
 #pragma unroll
 						for (int e = 0; e < 8; ++e)
 							if (c0 + c + e < R) {
-								if (MODE == TC_L2L) o[e] += v[e] + dg[c0 + c + e] * xs[c0 + c + e];
-								else if constexpr (F16) o[e] = v[e] * out_scale;
+								if constexpr (F16) o[e] = v[e] * out_scale;
 								else o[e] = v[e];
 							}
 					}
@@ -994,11 +976,11 @@ int row_map(Context& ctx, CUtensorMap* m, const void* base, uint64_t cols, uint6
 // block per item (the hardware's block scheduler hands them out).
 template <int NC, int NA, int SLOTS = M2L_SLOTS, int MODE = TC_M2L, bool F16 = false, bool TMA = false>
 int run_tc(Context& ctx, const M2LPlan& plan, const uint4* ops, const float* mult, float* loc, int R, int S, float* part,
-           bool timed, size_t src_cells, const float* diag = nullptr, int n_src = 0, bool persistent = true,
+           bool timed, size_t src_cells, int n_src = 0, bool persistent = true,
            const unsigned* bmax = nullptr, float t_inv = 1.f, const uint4* shi = nullptr, const uint4* slo = nullptr,
            const CUtensorMap* maps = nullptr)
 {
-	using C = TcCfg<NC, NA, MODE != TC_L2L && !TMA, F16>;
+	using C = TcCfg<NC, NA, !TMA, F16>;
 	CUtensorMap m_hi, m_lo;
 	std::memset(&m_hi, 0, sizeof(m_hi));
 	std::memset(&m_lo, 0, sizeof(m_lo));
@@ -1017,12 +999,12 @@ int run_tc(Context& ctx, const M2LPlan& plan, const uint4* ops, const float* mul
 	if (persistent)
 		m2l_tc_kernel<NC, NA, SLOTS, MODE, true, F16, TMA><<<grid, TC_THREADS, C::SMEM, ctx.stream>>>(
 			reinterpret_cast<const uint8_t*>(ops), mult, loc, plan.vtab, plan.order, plan.oct_count, R, part,
-			plan.cells, diag, ctx.dev_flags, tr, src_cells, MODE == TC_M2L ? 343 : 8, work, S, total, bmax, t_inv,
+			plan.cells, ctx.dev_flags, tr, src_cells, MODE == TC_M2L ? 343 : 8, work, S, total, bmax, t_inv,
 			shi, slo, m_hi, m_lo, (int)src_cells);
 	else
 		m2l_tc_kernel<NC, NA, SLOTS, MODE, false, F16, TMA><<<grid, TC_THREADS, C::SMEM, ctx.stream>>>(
 			reinterpret_cast<const uint8_t*>(ops), mult, loc, plan.vtab, plan.order, plan.oct_count, R, part,
-			plan.cells, diag, ctx.dev_flags, tr, src_cells, MODE == TC_M2L ? 343 : 8, work, S, total, bmax, t_inv,
+			plan.cells, ctx.dev_flags, tr, src_cells, MODE == TC_M2L ? 343 : 8, work, S, total, bmax, t_inv,
 			shi, slo, m_hi, m_lo, (int)src_cells);
 	if (timed) {
 		LFMM_CUDA(ctx, cudaEventRecord(ctx.kev[ctx.kev_used + 1], ctx.stream));
@@ -1112,7 +1094,7 @@ int launch_tc(Context& ctx, const M2LPlan& plan, const uint4* ops, const float* 
 			for (int cand = 1; cand <= maxS; cand *= 2) {
 				LFMM_CUDA(ctx, cudaEventRecord(e0, ctx.stream));
 				int st = run_tc<NC, NA, M2L_SLOTS, TC_M2L, F16, TMA>(ctx, plan, ops, mult, loc, R, cand, part, false,
-				                                                     plan.cells, nullptr, n_src, mode == 0, bmax, t_inv,
+				                                                     plan.cells, n_src, mode == 0, bmax, t_inv,
 				                                                     shi, slo, TMA ? maps : nullptr);
 				if (st) return st;
 				LFMM_CUDA(ctx, cudaEventRecord(e1, ctx.stream));
@@ -1128,28 +1110,18 @@ int launch_tc(Context& ctx, const M2LPlan& plan, const uint4* ops, const float* 
 		pers = bestP;
 	}
 	return run_tc<NC, NA, M2L_SLOTS, TC_M2L, F16, TMA>(ctx, plan, ops, mult, loc, R, S, part, true, plan.cells,
-	                                                   nullptr, n_src, pers, bmax, t_inv, shi, slo,
+	                                                   n_src, pers, bmax, t_inv, shi, slo,
 	                                                   TMA ? maps : nullptr);
 }
 
-// M2M (8 slots, stored) or L2L (1 slot, added) of one level: S = 1.
+// M2M (8 slots, stored) of one level: S = 1.
 template <int NC, int NA>
-int launch_shift_tc(Context& ctx, int mode, const M2LPlan& plan, const uint4* ops, const float* src, float* dst, int R,
-                    size_t src_cells)
+int launch_m2m_tc(Context& ctx, const M2LPlan& plan, const uint4* ops, const float* src, float* dst, int R,
+                  size_t src_cells)
 {
-	using C = TcCfg<NC, NA>;
-	using CL = TcCfg<NC, NA, false>;
-	if (mode == TC_M2M) {
-		LFMM_CUDA(ctx, cudaFuncSetAttribute(m2l_tc_kernel<NC, NA, 8, TC_M2M, false, false, false>,
-		                                    cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-		return run_tc<NC, NA, 8, TC_M2M>(ctx, plan, ops, src, dst, R, 1, nullptr, false, src_cells, nullptr, 0,
-		                                 false);
-	}
-	LFMM_CUDA(ctx, cudaFuncSetAttribute(m2l_tc_kernel<NC, NA, 1, TC_L2L, false, false, false>,
-	                                    cudaFuncAttributeMaxDynamicSharedMemorySize, CL::SMEM));
-	// the diagonal [8][NC] follows the 8 operators
-	const float* diag = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(ops) + 8 * C::DIR_BYTES);
-	return run_tc<NC, NA, 1, TC_L2L>(ctx, plan, ops, src, dst, R, 1, nullptr, false, src_cells, diag, 0, false);
+	LFMM_CUDA(ctx, cudaFuncSetAttribute(m2l_tc_kernel<NC, NA, 8, TC_M2M, false, false, false>,
+	                                    cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<NC, NA>::SMEM));
+	return run_tc<NC, NA, 8, TC_M2M>(ctx, plan, ops, src, dst, R, 1, nullptr, false, src_cells, 0, false);
 }
 
 std::mutex g_upload_mu;
@@ -1258,15 +1230,14 @@ int tc_ops_convert(Context& ctx, const double* ops64, int ndir, int N, void* out
 #define LFMM_TC_ORDERS(X) X(64, 64) X(80, 80) X(96, 96) X(112, 112) X(144, 144) X(160, 160) \
 	X(192, 160) X(224, 160) X(240, 160) X(272, 160) X(320, 160) X(352, 160)
 
-int shift_gemm_tc(Context& ctx, int mode, const M2LPlan& plan, const uint4* ops, const float* src, float* dst, int N,
-                  size_t src_cells)
+int m2m_gemm_tc(Context& ctx, const M2LPlan& plan, const uint4* ops, const float* src, float* dst, int N,
+                size_t src_cells)
 {
-	if (mode != TC_M2M && mode != TC_L2L) { ctx.last_error = "tensor-core shift: bad mode"; return ERR_ARG; }
 	const int R = N * (N + 1), NC = m2l_padded(N), NA = m2l_tc_drained(N);
-#define LFMM_TC_SHIFT(nc, na) if (NC == nc && NA == na) return launch_shift_tc<nc, na>(ctx, mode, plan, ops, src, dst, R, src_cells);
-	LFMM_TC_ORDERS(LFMM_TC_SHIFT)
-#undef LFMM_TC_SHIFT
-	ctx.last_error = "tensor-core shift: unsupported order";
+#define LFMM_TC_M2M(nc, na) if (NC == nc && NA == na) return launch_m2m_tc<nc, na>(ctx, plan, ops, src, dst, R, src_cells);
+	LFMM_TC_ORDERS(LFMM_TC_M2M)
+#undef LFMM_TC_M2M
+	ctx.last_error = "tensor-core M2M: unsupported order";
 	return ERR_UNSUPPORTED;
 }
 

@@ -100,14 +100,12 @@ __device__ __forceinline__ void rotate_y_t(const typename V2<real>::t* __restric
 	}
 }
 
-enum { SOP_M2M = 0, SOP_L2L = 1 };
-
-// Scaled M2M / L2L along one of the 8 diagonal offsets (warp-cooperative).
-template <int OP, typename real>
-__device__ void translate_scaled(const typename V2<real>::t* __restrict__ src, int dirid,
-                                 typename V2<real>::t (&acc)[CMAX], int N, int Nx2, SmemT<real>& sm,
-                                 const Tab<real>& T, unsigned* flags)
+// Scaled M2M from one of the 8 children (warp-cooperative), FP64: builds the
+// dense operators.
+__device__ inline void translate_scaled(const double2* __restrict__ src, int dirid, double2 (&acc)[CMAX], int N,
+                                        int Nx2, SmemT<double>& sm, const Tab<double>& T, unsigned* flags)
 {
+	using real = double;
 	const int lane = threadIdx.x & 31;
 	int4 di = T.dirinfo[dirid];
 	if (di.x < 0 || di.y < 0 || di.z < 0 || di.w < 0) {
@@ -118,8 +116,7 @@ __device__ void translate_scaled(const typename V2<real>::t* __restrict__ src, i
 	const real* D2 = T.dmat + (size_t)di.y * dsize(MAXN3);
 	const typename V2<real>::t* E1 = T.emat + di.z * MAXN3;
 	const typename V2<real>::t* E2 = T.emat + di.w * MAXN3;
-	// M2M: rho / h_child = sqrt(3)/2 ; L2L: rho / h_parent = sqrt(3)/4
-	const double rho = OP == SOP_M2M ? 0.86602540378443864676 : 0.43301270189221932338;
+	const double rho = 0.86602540378443864676;     // rho / h_child = sqrt(3) / 2
 	for (int i = lane; i < N; i += 32) {
 		double p = 1.0;
 		for (int j = 0; j < i; ++j) p *= rho;
@@ -133,7 +130,7 @@ __device__ void translate_scaled(const typename V2<real>::t* __restrict__ src, i
 	__syncwarp();
 	rotate_y_t<real>(sm.a, sm.b, D1, Nx2);
 	__syncwarp();
-	const real* cube = OP == SOP_M2M ? T.m2m : T.l2l;
+	const real* cube = T.m2m;
 #pragma unroll
 	for (int t = 0; t < CMAX; ++t) {
 		int c = lane + 32 * t;
@@ -141,23 +138,13 @@ __device__ void translate_scaled(const typename V2<real>::t* __restrict__ src, i
 			const int j = tri_row(c), k = c - tix(j, 0);
 			const real* cf = cube + (j * MAXN3 + k) * MAXN3;
 			real sr = 0, si = 0;
-			if (OP == SOP_M2M) {
-				for (int n = 0; j - n >= k; ++n) {
-					real f = cf[n] * sm.rn[n];
-					typename V2<real>::t w = sm.b[tix(j - n, k)];
-					sr = fma(f, w.x, sr); si = fma(f, w.y, si);
-				}
-				real s = (real)ldexp(1.0, -j);
-				sr *= s; si *= s;
-			} else {
-				for (int n = j; n < N; ++n) {
-					real f = cf[n] * sm.rn[n - j];
-					typename V2<real>::t w = sm.b[tix(n, k)];
-					sr = fma(f, w.x, sr); si = fma(f, w.y, si);
-				}
-				real s = (real)ldexp(1.0, -(j + 1));
-				sr *= s; si *= s;
+			for (int n = 0; j - n >= k; ++n) {
+				real f = cf[n] * sm.rn[n];
+				typename V2<real>::t w = sm.b[tix(j - n, k)];
+				sr = fma(f, w.x, sr); si = fma(f, w.y, si);
 			}
+			const real s = ldexp(1.0, -j);
+			sr *= s; si *= s;
 			sm.a[c] = V2<real>::make(sr, si);
 		}
 	}
@@ -173,65 +160,6 @@ __device__ void translate_scaled(const typename V2<real>::t* __restrict__ src, i
 		}
 	}
 	__syncwarp();
-}
-
-// parent (level L, array par) = sum of scaled M2M from its children (level L+1, array chi)
-template <typename real>
-__global__ void __launch_bounds__(WPB * 32) m2m_scaled_kernel(DevTree t, int L, const typename V2<real>::t* __restrict__ chi,
-                                                              typename V2<real>::t* __restrict__ par, int N,
-                                                              Tab<real> T, unsigned* flags)
-{
-	__shared__ SmemT<real> sm[WPB];
-	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-	size_t c = (size_t)blockIdx.x * WPB + w;
-	if (c >= t.lsize[L]) return;
-	const int Nx2 = N * (N + 1) / 2;
-	size_t g = t.loff[L] + c, cb = t.loff[L + 1];
-	if (t.beg[g] >= t.end[g]) return;     // a leaf keeps its P2M expansion
-	typename V2<real>::t acc[CMAX];
-#pragma unroll
-	for (int k = 0; k < CMAX; ++k) acc[k] = V2<real>::make(0, 0);
-	for (uint32_t k = t.beg[g]; k < t.end[g]; ++k) {
-		uint64_t oct = t.code[cb + k] & 7ull;
-		int d = dir_id(2 * (int)((oct >> 2) & 1) - 1, 2 * (int)((oct >> 1) & 1) - 1, 2 * (int)(oct & 1) - 1);
-		translate_scaled<SOP_M2M, real>(chi + (size_t)k * Nx2, d, acc, N, Nx2, sm[w], T, flags);
-	}
-	typename V2<real>::t* out = par + c * Nx2;
-#pragma unroll
-	for (int k = 0; k < CMAX; ++k) {
-		int cc = lane + 32 * k;
-		if (cc < Nx2) out[cc] = acc[k];
-	}
-}
-
-// child (level L, array chi) += scaled L2L from its parent (level L-1, array par)
-template <typename real>
-__global__ void __launch_bounds__(WPB * 32) l2l_scaled_kernel(DevTree t, int L, const typename V2<real>::t* __restrict__ par,
-                                                              typename V2<real>::t* __restrict__ chi, int N,
-                                                              Tab<real> T, unsigned* flags)
-{
-	__shared__ SmemT<real> sm[WPB];
-	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-	size_t c = (size_t)blockIdx.x * WPB + w;
-	if (c >= t.lsize[L]) return;
-	const int Nx2 = N * (N + 1) / 2;
-	size_t g = t.loff[L] + c;
-	int32_t p = t.parent[g];
-	typename V2<real>::t* out = chi + c * Nx2;
-	typename V2<real>::t acc[CMAX];
-#pragma unroll
-	for (int k = 0; k < CMAX; ++k) {
-		int cc = lane + 32 * k;
-		acc[k] = cc < Nx2 ? out[cc] : V2<real>::make(0, 0);
-	}
-	uint64_t oct = t.code[g] & 7ull;
-	int d = dir_id(1 - 2 * (int)((oct >> 2) & 1), 1 - 2 * (int)((oct >> 1) & 1), 1 - 2 * (int)(oct & 1));
-	translate_scaled<SOP_L2L, real>(par + (size_t)p * Nx2, d, acc, N, Nx2, sm[w], T, flags);
-#pragma unroll
-	for (int k = 0; k < CMAX; ++k) {
-		int cc = lane + 32 * k;
-		if (cc < Nx2) out[cc] = acc[k];
-	}
 }
 
 template <typename real> __device__ __forceinline__ real rsq(real x);
@@ -473,12 +401,6 @@ __device__ void eval_expansion(const typename V2<real>::t* __restrict__ Lc, real
 	fz = mt0 * x - mt1 * y;
 }
 
-template <typename real>
-__global__ void convert_kernel(const real* __restrict__ in, double* __restrict__ out, size_t n)
-{
-	size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < n) out[i] = (double)in[i];
-}
 template <typename real>
 __global__ void convert_back_kernel(const double* __restrict__ in, real* __restrict__ out, size_t n)
 {

@@ -9,6 +9,7 @@
 // generated on the GPU in FP64 from that canonical angle with the reference's
 // three-stage recurrence (special_functions.cpp:211-351).
 #include "context.cuh"
+#include "rot.cuh"
 #include <cmath>
 #include <map>
 
@@ -100,6 +101,25 @@ __global__ void exp_kernel(const double* __restrict__ phis, int nslots, double2*
 	out[slot * MAXN3 + m] = make_double2(cos(a), sin(a));
 }
 
+// Rotation about y of the (n, m >= 0) coefficients, per degree n: real parts
+// through D[m,k] + D[m,-k], imaginary parts through D[m,k] - D[m,-k] (D[m,0]
+// for k = 0), laid out as MMA fragments, zero past the block.
+__global__ void rot_frag_kernel(const double* __restrict__ dmat, double2* __restrict__ out)
+{
+	const int f = blockIdx.x, lane = threadIdx.x;
+	const double* D = dmat + (size_t)blockIdx.y * dsize(MAXN3);
+	int n = 0;
+	while (rot_frag0(n + 1) <= f) ++n;
+	const int K = rot_ksteps(n), kt = (f - rot_frag0(n)) % K, mt = (f - rot_frag0(n)) / K;
+	const int m = 8 * mt + (lane >> 2), k = 4 * kt + (lane & 3);
+	double2 v = make_double2(0.0, 0.0);
+	if (m <= n && k <= n) {
+		const double* r = D + dix(n, m, 0);
+		v = k == 0 ? make_double2(r[0], r[0]) : make_double2(r[k] + r[-k], r[k] - r[-k]);
+	}
+	out[((size_t)blockIdx.y * rot_frag0(MAXN3) + f) * 32 + lane] = v;
+}
+
 } // namespace
 
 int tables_build(Context& ctx)
@@ -187,6 +207,8 @@ int tables_build(Context& ctx)
 	LFMM_CUDA(ctx, cudaMemcpyAsync(T.l2l, l2l.data(), sizeof(double) * C, cudaMemcpyHostToDevice, s));
 	wignerd_kernel<<<T.n_dslots, 32, 0, s>>>(d_th, T.n_dslots, T.dmat);
 	exp_kernel<<<T.n_eslots, 32, 0, s>>>(d_ph, T.n_eslots, T.emat);
+	LFMM_CUDA(ctx, cudaMalloc(&T.rotf, sizeof(double2) * 32 * rot_frag0(MAXN3) * (size_t)T.n_dslots));
+	rot_frag_kernel<<<dim3(rot_frag0(MAXN3), T.n_dslots), 32, 0, s>>>(T.dmat, T.rotf);
 	LFMM_CUDA(ctx, cudaGetLastError());
 	// FP32 copies (mixed form)
 	size_t nd = (size_t)dsize(MAXN3) * T.n_dslots, ne = (size_t)2 * MAXN3 * T.n_eslots;
@@ -213,7 +235,7 @@ int tables_build(Context& ctx)
 void tables_free(Tables& TH)
 {
 	DevTables& T = TH.d;
-	cudaFree(T.dmat); cudaFree(T.emat); cudaFree(T.dirinfo); cudaFree(T.knm);
+	cudaFree(T.dmat); cudaFree(T.rotf); cudaFree(T.emat); cudaFree(T.dirinfo); cudaFree(T.knm);
 	cudaFree(T.m2l); cudaFree(T.m2m); cudaFree(T.l2l);
 	cudaFree(T.dmat_f); cudaFree(T.emat_f); cudaFree(T.knm_f);
 	cudaFree(T.m2l_f); cudaFree(T.m2m_f); cudaFree(T.l2l_f);
