@@ -56,13 +56,6 @@ struct DevTables {
 	double* m2l = nullptr;
 	double* m2m = nullptr;
 	double* l2l = nullptr;
-	// FP32 copies for the mixed form (same layouts)
-	float* dmat_f = nullptr;
-	float2* emat_f = nullptr;
-	float* knm_f = nullptr;
-	float* m2l_f = nullptr;
-	float* m2m_f = nullptr;
-	float* l2l_f = nullptr;
 };
 
 struct Tables {

@@ -4,10 +4,12 @@
 // Passes: P2M (every leaf, any level) -> M2M -> M2L (V) ->
 // P2L (X) -> L2L -> leaves: P2P (self + U), M2P (W), L2P.
 #include <cmath>
-#include "scaled_kernels.cuh"
+#include "far_kernels.cuh"
 #include "m2l_tc.cuh"
 #include "rot.cuh"
 #include <algorithm>
+#include <mutex>
+#include <type_traits>
 
 namespace lfmm {
 
@@ -15,51 +17,54 @@ using namespace scaled;
 
 namespace {
 
+std::mutex g_const_mu;
 bool g_scaled_const_ready[64] = {};
 
 int upload_scaled_constants(Context& ctx)
 {
+	std::lock_guard<std::mutex> lock(g_const_mu);
 	if (ctx.device < 0 || ctx.device >= 64) { ctx.last_error = "device index above 63"; return ERR_ARG; }
 	if (g_scaled_const_ready[ctx.device]) return OK;
 	float2 rec_f[NXD];
 	double2 rec_d[NXD];
-	float sig_f[MAXN3 + 2];
-	double sig_d[MAXN3 + 2];
+	GradF grad_f[2][NXD];
+	GradD grad_d[2][NXD];
 	for (int n = 0; n <= MAXN3; ++n)
 		for (int m = 0; m <= n; ++m) {
 			const int i = tix(n, m);
 			const double d1 = (double)(n + 1) * (n + 1) - (double)m * m;
 			rec_d[i] = make_double2((2.0 * n + 1.0) / std::sqrt(d1), std::sqrt(((double)n * n - (double)m * m) / d1));
 			rec_f[i] = make_float2((float)rec_d[i].x, (float)rec_d[i].y);
+			const double z[2] = {(n + 1.0 - m) * (n + 1 + m), std::max((n - m) * (n + m), 0) * 1.0};
+			const double p[2] = {(n + 2.0 - m) * (n + 1 - m), std::max((n + m - 1) * (n + m), 0) * 1.0};
+			const double q[2] = {(n + 2.0 + m) * (n + 1 + m), std::max((n - m - 1) * (n - m), 0) * 1.0};
+			for (int k = 0; k < 2; ++k) {
+				grad_d[k][i] = GradD{std::sqrt(z[k]), std::sqrt(p[k]), std::sqrt(q[k]), n | m << 8};
+				grad_f[k][i] = GradF{(float)grad_d[k][i].z, (float)grad_d[k][i].p, (float)grad_d[k][i].m, n | m << 8};
+			}
 		}
-	sig_d[0] = 0.0;
-	for (int m = 1; m <= MAXN3 + 1; ++m) sig_d[m] = -std::sqrt((2.0 * m - 1.0) / (2.0 * m));
-	for (int m = 0; m <= MAXN3 + 1; ++m) sig_f[m] = (float)sig_d[m];
-	float inv_f[NINV];
-	double inv_d[NINV];
-	inv_f[0] = 0.f; inv_d[0] = 0.0;
-	for (int k = 1; k < NINV; ++k) { inv_d[k] = 1.0 / k; inv_f[k] = 1.0f / (float)k; }
-	LFMM_CUDA(ctx, cudaMemcpyToSymbol(c_inv_f, inv_f, sizeof(inv_f)));
-	LFMM_CUDA(ctx, cudaMemcpyToSymbol(c_inv_d, inv_d, sizeof(inv_d)));
-	LFMM_CUDA(ctx, cudaMemcpyToSymbol(c_rec_f, rec_f, sizeof(rec_f)));
-	LFMM_CUDA(ctx, cudaMemcpyToSymbol(c_rec_d, rec_d, sizeof(rec_d)));
-	LFMM_CUDA(ctx, cudaMemcpyToSymbol(c_sig_f, sig_f, sizeof(sig_f)));
-	LFMM_CUDA(ctx, cudaMemcpyToSymbol(c_sig_d, sig_d, sizeof(sig_d)));
+	double S_d[MAXN3 + 1];
+	float S_f[MAXN3 + 1];
+	S_d[0] = 1.0;
+	for (int m = 1; m <= MAXN3; ++m) S_d[m] = -S_d[m - 1] * std::sqrt((2.0 * m - 1.0) / (2.0 * m));
+	for (int m = 0; m <= MAXN3; ++m) S_f[m] = (float)S_d[m];
+	LFMM_CUDA(ctx, cudaMemcpyToSymbol(g_rec_f, rec_f, sizeof(rec_f)));
+	LFMM_CUDA(ctx, cudaMemcpyToSymbol(g_rec_d, rec_d, sizeof(rec_d)));
+	LFMM_CUDA(ctx, cudaMemcpyToSymbol(g_grad_f, grad_f, sizeof(grad_f)));
+	LFMM_CUDA(ctx, cudaMemcpyToSymbol(g_grad_d, grad_d, sizeof(grad_d)));
+	LFMM_CUDA(ctx, cudaMemcpyToSymbol(g_S_f, S_f, sizeof(S_f)));
+	LFMM_CUDA(ctx, cudaMemcpyToSymbol(g_S_d, S_d, sizeof(S_d)));
 	g_scaled_const_ready[ctx.device] = true;
 	return OK;
 }
 
-template <typename real> Tab<real> tables_of(const DevTables& T);
-template <> Tab<double> tables_of<double>(const DevTables& T) { return Tab<double>{T.dmat, T.emat, T.m2m, T.l2l, T.knm, T.dirinfo}; }
-template <> Tab<float> tables_of<float>(const DevTables& T) { return Tab<float>{T.dmat_f, T.emat_f, T.m2m_f, T.l2l_f, T.knm_f, T.dirinfo}; }
-
 // Dense FP64 scaled M2M operators, one per child octant o (the octant bits
 // of the child's code): column r is translate_scaled applied to the r-th unit
 // vector.  out: [8][MT][MT], pre-zeroed.
-__global__ void __launch_bounds__(WPB * 32) m2m_ops_kernel(int N, int MT, Tab<double> T, double* __restrict__ out,
+__global__ void __launch_bounds__(WPB * 32) m2m_ops_kernel(int N, int MT, DevTables T, double* __restrict__ out,
                                                            unsigned* flags)
 {
-	__shared__ SmemT<double> sm[WPB];
+	__shared__ ShiftSmem sm[WPB];
 	__shared__ double2 unit[WPB][NX2MAX];
 	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 	const int Nx2 = N * (N + 1) / 2, R = 2 * Nx2;
@@ -109,7 +114,7 @@ const uint4* m2m_ops_tc(Context& ctx, int N, int& st)
 		return nullptr;
 	}
 	cudaMemsetAsync(d, 0, bytes64, ctx.stream);
-	m2m_ops_kernel<<<div_up((size_t)8 * R, WPB), WPB * 32, 0, ctx.stream>>>(N, MT, tables_of<double>(ctx.tables.d), d,
+	m2m_ops_kernel<<<div_up((size_t)8 * R, WPB), WPB * 32, 0, ctx.stream>>>(N, MT, ctx.tables.d, d,
 	                                                                        ctx.dev_flags);
 	st = cudaGetLastError() == cudaSuccess ? tc_ops_convert(ctx, d, 8, N, tc) : ERR_CUDA;
 	if (cudaStreamSynchronize(ctx.stream) != cudaSuccess) st = ERR_CUDA;
@@ -137,6 +142,16 @@ const uint4* m2m_ops_tc(Context& ctx, int N, int& st)
 // 281 at 32,768.
 constexpr size_t ROT_M2L_CELLS = 512, ROT_M2M_CELLS = 6144;
 
+// Instances of the chain kernels by the steps of their busiest lane.
+template <typename F>
+void by_steps(int N, F go)
+{
+	if (N <= 8) go(std::integral_constant<int, 8>());
+	else if (N <= 12) go(std::integral_constant<int, 12>());
+	else if (N <= 16) go(std::integral_constant<int, 17>());
+	else go(std::integral_constant<int, 23>());
+}
+
 template <typename real>
 int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, SolveStats* stats,
             const int* level_N)
@@ -145,17 +160,11 @@ int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, S
 	cudaStream_t s = ctx.stream;
 	const bool timing = ctx.timing != 0;
 	const int Nx2 = N * (N + 1) / 2, R = 2 * Nx2;
-	const size_t n = t.n, C = t.ncells;
-	const Tab<real> T = tables_of<real>(ctx.tables.d);
-	const real* knm = T.knm;
-	real* xr = static_cast<real*>(ctx.arena.take(sizeof(real) * n));
-	real* yr = static_cast<real*>(ctx.arena.take(sizeof(real) * n));
-	real* zr = static_cast<real*>(ctx.arena.take(sizeof(real) * n));
-	real* qr = static_cast<real*>(ctx.arena.take(sizeof(real) * n));
+	const size_t C = t.ncells;
 	v2* outer = static_cast<v2*>(ctx.arena.take(sizeof(v2) * C * Nx2));
 	v2* inner = static_cast<v2*>(ctx.arena.take(sizeof(v2) * C * Nx2));
 	const bool coarse64 = sizeof(real) == sizeof(float);
-	if (!xr || !yr || !zr || !qr || !outer || !inner) {
+	if (!outer || !inner) {
 		ctx.last_error = "scaled solve: allocation failed";
 		return ERR_OOM;
 	}
@@ -164,10 +173,12 @@ int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, S
 	LFMM_CUDA(ctx, cudaMemsetAsync(field, 0, sizeof(double) * 3 * n_out, s));
 	LFMM_CUDA(ctx, cudaMemsetAsync(outer, 0, sizeof(v2) * C * Nx2, s));
 	LFMM_CUDA(ctx, cudaMemsetAsync(inner, 0, sizeof(v2) * C * Nx2, s));
-	const unsigned nl = (unsigned)t.nleaves;
-	relcoords_kernel<real><<<nl, 128, 0, s>>>(t, xr, yr, zr, qr);
+	const unsigned resident = 8u * (unsigned)ctx.num_sms;
 	if (t.depth > 2)                       // multipoles below level 2 reach nothing
-		p2m_scaled_kernel<real><<<div_up(nl, WPB), WPB * 32, 0, s>>>(t, xr, yr, zr, qr, N, knm, outer);
+		by_steps(N, [&](auto st_) {
+			p2m_scaled_kernel<real, decltype(st_)::value>
+				<<<std::min(div_up(t.nleaves, FWPB), resident), FWPB * 32, 0, s>>>(t, N, outer);
+		});
 	int st;
 	// the tensor-core engine on the FP32 expansions' larger levels (M2L; M2M
 	// through dense scaled operators, one per child octant)
@@ -223,8 +234,20 @@ int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, S
 			}
 		}
 	}
-	if (t.adaptive && t.n_x > 0)
-		p2l_kernel<real><<<div_up(C, WPB), WPB * 32, 0, s>>>(t, N, knm, inner);
+	if (t.adaptive && t.n_x > 0) {
+		// counter, list of longs, list of shorts (at most one cell per entry)
+		const size_t nlong = t.n_x / FAR_SHORT + 1;
+		uint32_t* next = static_cast<uint32_t*>(ctx.arena.take(sizeof(uint32_t) * (nlong + t.n_x + 3)));
+		if (!next) { ctx.last_error = "scaled solve: allocation failed"; return ERR_OOM; }
+		uint32_t *longs = next + 1, *shorts = longs + 1 + nlong;
+		LFMM_CUDA(ctx, cudaMemsetAsync(next, 0, 2 * sizeof(uint32_t), s));
+		LFMM_CUDA(ctx, cudaMemsetAsync(shorts, 0, sizeof(uint32_t), s));
+		x_select_kernel<<<div_up(C, 256), 256, 0, s>>>(t, shorts, longs);
+		by_steps(N, [&](auto st_) {
+			p2l_kernel<real, decltype(st_)::value><<<resident, FWPB * 32, 0, s>>>(t, N, inner, next, shorts);
+			p2l_long_kernel<real, decltype(st_)::value><<<2 * ctx.num_sms, FWL * 32, 0, s>>>(t, N, inner, longs);
+		});
+	}
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[3], s));
 	for (int L = 3; L < t.depth; ++L) {
 		if (t.lsize[L] == 0) continue;
@@ -235,22 +258,23 @@ int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, S
 		if (st) return st;
 	}
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[4], s));
-	if constexpr (sizeof(real) == sizeof(float)) {
-		// the near field (a resident grid taking leaves from a counter), then
-		// the expansions added onto it
-		constexpr int LWP = 4, LWE = eval_warps<real>();
-		unsigned* next_leaf = static_cast<unsigned*>(ctx.arena.take(sizeof(unsigned)));
-		if (!next_leaf) { ctx.last_error = "scaled solve: allocation failed"; return ERR_OOM; }
-		LFMM_CUDA(ctx, cudaMemsetAsync(next_leaf, 0, sizeof(unsigned), s));
-		p2p_f32_kernel<LWP><<<6 * ctx.num_sms, LWP * 32, 0, s>>>(t, qr, pot, field, next_leaf);
-		unsigned* next_eval = static_cast<unsigned*>(ctx.arena.take(sizeof(unsigned)));
-		if (!next_eval) { ctx.last_error = "scaled solve: allocation failed"; return ERR_OOM; }
-		LFMM_CUDA(ctx, cudaMemsetAsync(next_eval, 0, sizeof(unsigned), s));
-		eval_scaled_kernel<real, LWE><<<8 * ctx.num_sms, LWE * 32, 0, s>>>(t, outer, inner, N, pot, field, next_eval);
-	} else {
-		constexpr int LW = leaf_warps<real>();
-		leaves_scaled_kernel<real><<<div_up(nl, LW), LW * 32, 0, s>>>(t, qr, outer, inner, N, knm, pot, field);
-	}
+	// the near field, then the expansions added onto it: resident grids taking
+	// leaves from a counter
+	uint32_t* next = static_cast<uint32_t*>(ctx.arena.take(sizeof(uint32_t) * (5 + t.n_w / FAR_SHORT)));
+	if (!next) { ctx.last_error = "scaled solve: allocation failed"; return ERR_OOM; }
+	uint32_t* longs = next + 3;
+	LFMM_CUDA(ctx, cudaMemsetAsync(next, 0, 4 * sizeof(uint32_t), s));
+	constexpr int LWP = 4;
+	if constexpr (sizeof(real) == sizeof(float))
+		p2p_f32_kernel<LWP><<<6 * ctx.num_sms, LWP * 32, 0, s>>>(t, pot, field, next);
+	else
+		p2p_f64_kernel<LWP><<<resident, LWP * 32, 0, s>>>(t, pot, field, next);
+	const size_t sm_e = eval_smem<real>(FWPB, N), sm_l = eval_smem<real>(FWL, N);
+	LFMM_CUDA(ctx, cudaFuncSetAttribute(eval_scaled_kernel<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_e));
+	LFMM_CUDA(ctx, cudaFuncSetAttribute(eval_long_kernel<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_l));
+	eval_scaled_kernel<real><<<resident, FWPB * 32, sm_e, s>>>(t, outer, inner, N, pot, field, next + 1, longs);
+	if (t.n_w > FAR_SHORT)
+		eval_long_kernel<real><<<2 * ctx.num_sms, FWL * 32, sm_l, s>>>(t, outer, inner, N, pot, field, next + 2, longs);
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[5], s));
 	LFMM_CUDA(ctx, cudaGetLastError());
 	(void)stats;
