@@ -81,6 +81,18 @@ __device__ __forceinline__ double rsqrt_refined(double x)
 	return fma(y * r, fma(r, 0.375, 0.5), y);
 }
 
+// 1 / x, x > 0: the hardware's FP64 reciprocal approximation refined by the
+// geometric series 1 / (1 - e) = 1 + e + e^2 + ..., e = 1 - x y (a seed error
+// below 2^-18 leaves e^3 < 2^-54).  The FP64 divide above 1e300.
+__device__ __forceinline__ double recip_refined(double x)
+{
+	if (!(x < 1e300)) return 1.0 / x;
+	double y;
+	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+	const double e = fma(-x, y, 1.0);
+	return fma(y, fma(e, e, e), y);
+}
+
 // Spherical coordinates with the reference's conventions
 // (common/simple_math.h:101-117): r gets +1e-12, phi = 0 on the z-axis,
 // +-pi/2 when |x| < 1e-12.

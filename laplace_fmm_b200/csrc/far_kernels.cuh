@@ -793,5 +793,135 @@ __global__ void __launch_bounds__(LW * 32) p2p_f64_kernel(DevTree t, double* __r
 	}
 }
 
+// ---- leaves of the plain form ----------------------------------------------
+// (uniform tree, unscaled expansions; the same harmonics at the reference's
+// points)
+
+// P2M: one warp per leaf.
+template <int STEPS>
+__global__ void __launch_bounds__(FWPB * 32) p2m_plain_kernel(DevTree t, int N, double2* __restrict__ outer)
+{
+	__shared__ ChainTab<double> tb;
+	chain_tab_fill(tb, N, threadIdx.x, FWPB * 32);
+	__syncthreads();
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, l = lane % CHL, LL = t.depth - 1;
+	const int Nx2 = N * (N + 1) / 2, T = chain_steps(N);
+	const size_t leaf = (size_t)blockIdx.x * FWPB + w;
+	if (leaf >= t.lsize[LL]) return;
+	const size_t g = t.loff[LL] + leaf;
+	const double cx = t.cx[g], cy = t.cy[g], cz = t.cz[g];
+	const uint32_t e = t.end[g];
+	ChainAcc<double, STEPS> A;
+	A.clear();
+	for (uint32_t base = t.beg[g]; base < e; base += 32) {
+		const uint32_t i = base + lane;
+		double q = 0, x = 0, y = 0, z = 0;
+		if (i < e) {
+			q = t.q[i]; x = t.x[i] - cx; y = t.y[i] - cy; z = t.z[i] - cz;
+			reference_point(x, y, z);
+		}
+		chain_add32<false, double, STEPS>(A, tb, q, x, y, z, (int)min(32u, e - base), N);
+	}
+	chain_reduce<double, STEPS>(A, N);
+	if (lane < CHL) {
+#pragma unroll
+		for (int s = 0; s < STEPS; ++s) {
+			if (s >= T) break;
+			const int o = tb.out[s * CHL + l];
+			if (o >= 0) outer[g * Nx2 + o] = make_double2(A.a[s].x, -A.a[s].y);
+		}
+	}
+}
+
+// Near field and (FAR) local expansion of 32 targets of a leaf on a block of
+// eight warps: the warps take the staged 32-source tiles of the leaf and its
+// close cells in turn and every eighth order of the expansion; fewer than 17
+// targets share a tile's sources out between groups of lanes.  Chunks of 32
+// targets are spread over gridDim.y where the leaves alone would not fill the
+// GPU.  FP64 pipe bound (about 22 operations per pair).  Before (a block of 128
+// threads per leaf, thread = target, the reference's spherical form per
+// target): 8 leaves of 256 particles 565 us, 4,096 of 32 at N = 9 617 us, 512
+// of 157 (39 targets) at N = 18 368 us.
+template <bool FAR>
+__global__ void __launch_bounds__(FWL * 32, 2) leaves_plain_kernel(DevTree t, const double2* __restrict__ inner, int N,
+                                                                  double* __restrict__ pot_out,
+                                                                  double* __restrict__ fld_out)
+{
+	extern __shared__ __align__(16) unsigned char sm_eval[];
+	__shared__ double4 ss[FWL][32];
+	__shared__ double part[FWL][32][4];
+	const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, LL = t.depth - 1, R = (N + 1) * (N + 2) / 2;
+	CoefRow<double>* C = reinterpret_cast<CoefRow<double>*>(sm_eval);
+	double2* ab = reinterpret_cast<double2*>(C + R);
+	double* S = reinterpret_cast<double*>(ab + R);
+	const size_t off = t.loff[LL], g = off + blockIdx.x;
+	const bool tmode = t.targets_num > 0;
+	const uint32_t tb = tmode ? t.tbeg[g] : t.beg[g], te = tmode ? t.tend[g] : t.end[g];
+	if (tb + 32 * blockIdx.y >= te) return;
+	if (FAR) {
+		eval_tab_fill<double>(ab, S, N, tid, FWL * 32);
+		derive_coefs<false, double>(inner + g * (size_t)(N * (N + 1) / 2), N, C, tid, FWL * 32);
+	}
+	const int ncl = t.close_cnt[g];
+	const int32_t* cl = t.close_idx + g * t.close_stride;
+	const double cx = t.cx[g], cy = t.cy[g], cz = t.cz[g];
+	for (uint32_t t0 = tb + 32 * blockIdx.y; t0 < te; t0 += 32 * gridDim.y) {
+		const int np = (int)min(32u, te - t0);
+		int lt = 0;
+		while ((1 << lt) < np) ++lt;
+		const int ti = lane & ((1 << lt) - 1), ph = lane >> lt, G = 32 >> lt;
+		const uint32_t i = t0 + min(ti, np - 1);
+		const double xi = t.x[i], yi = t.y[i], zi = t.z[i];
+		double o[4] = {0.0, 0.0, 0.0, 0.0};
+		int turn = 0;
+		for (int e = -1; e < ncl; ++e) {
+			const size_t sc = e < 0 ? g : off + cl[e];
+			const uint32_t sb = t.beg[sc], se = t.end[sc];
+			for (uint32_t s0 = sb; s0 < se; s0 += 32) {
+				if ((turn++ & (FWL - 1)) != w) continue;
+				const int cnt = (int)min(32u, se - s0);
+				__syncwarp();
+				if (lane < cnt) {
+					const uint32_t j = s0 + lane;
+					ss[w][lane] = make_double4(t.x[j], t.y[j], t.z[j], t.q[j]);
+				}
+				__syncwarp();
+				for (int j = ph; j < cnt; j += G) {
+					const double4 s = ss[w][j];
+					const double dx = xi - s.x, dy = yi - s.y, dz = zi - s.z;
+					const double inv = rsqrt_refined(fmax(dx * dx + dy * dy + dz * dz, FORCE_EPS2));
+					const double qi = s.w * inv, qi3 = qi * inv * inv;
+					o[0] += qi;
+					o[1] = fma(dx, qi3, o[1]); o[2] = fma(dy, qi3, o[2]); o[3] = fma(dz, qi3, o[3]);
+				}
+			}
+		}
+		for (int s = 1 << lt; s < 32; s <<= 1)
+#pragma unroll
+			for (int k = 0; k < 4; ++k) o[k] += __shfl_xor_sync(0xffffffffu, o[k], s);
+		__syncthreads();                       // the rows are derived; the last chunk's sums are read
+		if (FAR) {
+			double x[1] = {xi - cx}, y[1] = {yi - cy}, z[1] = {zi - cz}, s[1][4];
+			reference_point(x[0], y[0], z[0]);
+			eval_chains<false, double, 1>(C, ab, S, x, y, z, N, w, FWL, s);
+			o[0] += s[0][0];
+#pragma unroll
+			for (int k = 1; k < 4; ++k) o[k] -= s[0][k];
+		}
+		if (ph == 0 && ti < np) {
+#pragma unroll
+			for (int k = 0; k < 4; ++k) part[w][ti][k] = o[k];
+		}
+		__syncthreads();
+		const int tt = tid >> 2, k = tid & 3;
+		if (tt < np) {
+			double v = 0.0;
+			for (int q = 0; q < FWL; ++q) v += part[q][tt][k];
+			const size_t r = t.orig[t0 + tt];
+			if (k == 0) pot_out[r] = v; else fld_out[3 * r + k - 1] = v;
+		}
+	}
+}
+
 } // namespace scaled
 } // namespace lfmm

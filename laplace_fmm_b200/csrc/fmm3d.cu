@@ -2,10 +2,10 @@
 //
 // Operators follow the reference's CPU solver (cpu/multipole3d.cpp): P2M
 // 20-49, rotate-z / rotate-y 51-113, M2M / M2L / L2L as rotate, z-translate,
-// rotate back 115-226, passes 228-412, P2P + L2P 855-1294.  Every kernel is
-// warp-per-box (P2M, M2M, M2L, L2L) or block-per-leaf (P2P + L2P); lanes own
-// expansion coefficients, per-box data is staged in shared memory, there are
-// no atomics and no per-thread local arrays.
+// rotate back 115-226, passes 228-412, P2P + L2P 855-1294.  The translations
+// run on the factored engine (rot.cu), the leaves on far_kernels.cuh; the
+// per-pair rotation kernels here (warp per box, lanes own coefficients) are the
+// LFMM_M2L=rotation engine and build the dense operators.
 #include "fmm3d.cuh"
 #include "m2l_gemm.cuh"
 #include "rot.cuh"
@@ -151,61 +151,6 @@ __device__ void translate_warp(const double2* __restrict__ src, double px, doubl
 	__syncwarp();
 }
 
-// ---------------------------------------------------------------- P2M
-__global__ void __launch_bounds__(WPB * 32) p2m_kernel(DevTree t, Exp E, const double* __restrict__ knm)
-{
-	__shared__ double2 sacc[WPB][NX2MAX];
-	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-	const int LL = t.depth - 1;
-	size_t leaf = (size_t)blockIdx.x * WPB + w;
-	if (leaf >= t.lsize[LL]) return;
-	size_t g = t.loff[LL] + leaf;
-	const int N = E.N, Nx2 = E.Nx2;
-	for (int c = lane; c < Nx2; c += 32) sacc[w][c] = make_double2(0.0, 0.0);
-	__syncwarp();
-	const double cx = t.cx[g], cy = t.cy[g], cz = t.cz[g];
-	const uint32_t b = t.beg[g], e = t.end[g];
-	for (uint32_t base = b; base < e; base += 32) {
-		uint32_t i = base + lane;
-		double q = 0.0, r = 1.0, th = 1.0, ph = 0.0;
-		if (i < e) {
-			q = t.q[i];
-			dec_to_sph(t.x[i] - cx, t.y[i] - cy, t.z[i] - cz, r, th, ph);
-		}
-		double y, x;
-		sincos(th, &y, &x);
-		double Pmm = 1.0, rpow = 1.0;
-		for (int m = 0; m < N; ++m) {
-			if (m > 0) { Pmm = Pmm * y * (1 - 2 * m); rpow *= r; }
-			double sm_, cm_;
-			sincos(m * ph, &sm_, &cm_);
-			// r^n: r^m at n = m (r^0 = 1), then one factor of r per degree
-			double Pn = Pmm, Pn1 = 0.0, rn = rpow;
-			for (int n = m; n < N; ++n) {
-				if (n > m) {
-					double Pnew = (n == m + 1) ? Pmm * x * (2 * n - 1)
-					                           : ((2 * n - 1) * x * Pn - (n + m - 1) * Pn1) / (n - m);
-					Pn1 = Pn; Pn = Pnew; rn *= r;
-				}
-				double vr, vi;
-				if (n == 0) { vr = q; vi = 0.0; }
-				else {
-					double f = q * rn * knm[tix(n, m)] * Pn;
-					vr = f * cm_; vi = -f * sm_;
-				}
-				vr = warp_sum(vr); vi = warp_sum(vi);
-				if (lane == 0) {
-					double2 a = sacc[w][tix(n, m)];
-					sacc[w][tix(n, m)] = make_double2(a.x + vr, a.y + vi);
-				}
-			}
-		}
-	}
-	__syncwarp();
-	double2* out = E.outer + g * Nx2;
-	for (int c = lane; c < Nx2; c += 32) out[c] = sacc[w][c];
-}
-
 // ---------------------------------------------------------------- M2M
 __global__ void __launch_bounds__(WPB * 32) m2m_kernel(DevTree t, Exp E, int L, DevTables T, unsigned* flags)
 {
@@ -297,115 +242,6 @@ __global__ void __launch_bounds__(WPB * 32) l2l_kernel(DevTree t, Exp E, int L, 
 	for (int k = 0; k < CMAX; ++k) {
 		int cc = lane + 32 * k;
 		if (cc < E.Nx2) out[cc] = acc[k];
-	}
-}
-
-// ---------------------------------------------------------------- P2P + L2P
-constexpr int LEAF_THREADS = 128;
-
-// Local expansion evaluated at one target (reference cpu/multipole3d.cpp:
-// 1152-1208): Legendre recurrence streamed degree by degree per order m,
-// potential and the spherical-gradient field, then the Cartesian transform.
-__device__ void l2p_eval(const double2* __restrict__ Lc, double dx, double dy, double dz, int N,
-                         const double* __restrict__ knm, double& pot, double& fx, double& fy, double& fz)
-{
-	double r, th, ph;
-	dec_to_sph(dx, dy, dz, r, th, ph);
-	double y, x;
-	sincos(th, &y, &x);
-	double phi = 0.0, mt0 = 0.0, mt1 = 0.0, mt2 = 0.0;
-	double Pmm = 1.0, rpow = 1.0 / r;
-	for (int m = 0; m < N; ++m) {
-		if (m > 0) { Pmm = Pmm * y * (1 - 2 * m); rpow *= r; }
-		double sm_, cm_;
-		sincos(m * ph, &sm_, &cm_);
-		const double mult = m ? 2.0 : 1.0;
-		double Pn = Pmm, Pn1 = 0.0, rn = rpow;
-		for (int n = m; n < N; ++n) {
-			double Pnext = (n == m) ? Pmm * x * (2 * n + 1)
-			                        : ((2 * n + 1) * x * Pn - (n + m) * Pn1) / (n + 1 - m);
-			double K = knm[tix(n, m)];
-			double Yr = Pn * cm_ * K, Yi = Pn * sm_ * K;
-			double2 Lnm = Lc[tix(n, m)];
-			double cr = Lnm.x * rn, ci = Lnm.y * rn;
-			double ycr = Yr * cr - Yi * ci;                       // Re(Y coef)
-			phi += mult * (r * ycr);
-			double g = K * ((1 - m + n) * Pnext - (n + 1) * x * Pn) / y;
-			double dthr = cm_ * g, dthi = sm_ * g;
-			mt0 -= mult * (n * ycr);
-			mt1 -= mult * (cr * dthr - ci * dthi);
-			mt2 -= mult * (cr * (-m * Yi) - ci * (m * Yr));
-			Pn1 = Pn; Pn = Pnext; rn *= r;
-		}
-	}
-	pot += phi;
-	double s2, c2;
-	sincos(ph, &s2, &c2);
-	const double s1 = y, c1 = x;
-	fx += mt0 * s1 * c2 + mt1 * c1 * c2 - mt2 * s2 / s1;
-	fy += mt0 * s1 * s2 + mt1 * c1 * s2 + mt2 * c2 / s1;
-	fz += mt0 * c1 - mt1 * s1;
-}
-
-// One block per leaf: targets of the leaf against the leaf's sources and
-// every close leaf's sources, staged through shared memory in tiles, then
-// L2P; results scattered to input order.  q / max(r, 1e-4) and
-// q (r_i - r_j) / max(r, 1e-4)^3 as reference common/avx.h:128-146.
-__global__ void __launch_bounds__(LEAF_THREADS) leaves_kernel(DevTree t, Exp E, const double* __restrict__ knm,
-                                                              double* __restrict__ pot_out,
-                                                              double* __restrict__ fld_out)
-{
-	__shared__ double sx[LEAF_THREADS], sy[LEAF_THREADS], sz[LEAF_THREADS], sq[LEAF_THREADS];
-	__shared__ double2 sL[NX2MAX];
-	const int LL = t.depth - 1;
-	size_t leaf = blockIdx.x;
-	if (leaf >= t.lsize[LL]) return;
-	size_t off = t.loff[LL], g = off + leaf;
-	const bool tmode = t.targets_num > 0;
-	const uint32_t tb = tmode ? t.tbeg[g] : t.beg[g];
-	const uint32_t te = tmode ? t.tend[g] : t.end[g];
-	if (tb >= te) return;
-	for (int c = threadIdx.x; c < E.Nx2; c += LEAF_THREADS) sL[c] = E.inner[g * E.Nx2 + c];
-	const int ncl = t.close_cnt[g];
-	const int32_t* cl = t.close_idx + g * t.close_stride;
-	const double cx = t.cx[g], cy = t.cy[g], cz = t.cz[g];
-	for (uint32_t t0 = tb; t0 < te; t0 += LEAF_THREADS) {
-		uint32_t i = t0 + threadIdx.x;
-		const bool valid = i < te;
-		double xi = 0.0, yi = 0.0, zi = 0.0;
-		if (valid) { xi = t.x[i]; yi = t.y[i]; zi = t.z[i]; }
-		double pot = 0.0, fx = 0.0, fy = 0.0, fz = 0.0;
-		for (int e = -1; e < ncl; ++e) {
-			size_t sc = e < 0 ? g : off + cl[e];
-			const uint32_t sb = t.beg[sc], se = t.end[sc];
-			for (uint32_t s0 = sb; s0 < se; s0 += LEAF_THREADS) {
-				const int cnt = min((uint32_t)LEAF_THREADS, se - s0);
-				__syncthreads();
-				if (threadIdx.x < cnt) {
-					uint32_t j = s0 + threadIdx.x;
-					sx[threadIdx.x] = t.x[j]; sy[threadIdx.x] = t.y[j]; sz[threadIdx.x] = t.z[j]; sq[threadIdx.x] = t.q[j];
-				}
-				__syncthreads();
-				if (valid) {
-					for (int j = 0; j < cnt; ++j) {
-						double dx = xi - sx[j], dy = yi - sy[j], dz = zi - sz[j];
-						double r2 = fmax(dx * dx + dy * dy + dz * dz, FORCE_EPS2);
-						double inv = rsqrt(r2);
-						double qi = sq[j] * inv;
-						double qi3 = qi * inv * inv;
-						pot += qi;
-						fx = fma(dx, qi3, fx); fy = fma(dy, qi3, fy); fz = fma(dz, qi3, fz);
-					}
-				}
-			}
-		}
-		__syncthreads();
-		if (valid) {
-			l2p_eval(sL, xi - cx, yi - cy, zi - cz, E.N, knm, pot, fx, fy, fz);
-			uint32_t o = t.orig[i];
-			pot_out[o] = pot;
-			fld_out[3 * (size_t)o] = fx; fld_out[3 * (size_t)o + 1] = fy; fld_out[3 * (size_t)o + 2] = fz;
-		}
 	}
 }
 
@@ -501,7 +337,7 @@ int fmm3d_solve_device(Context& ctx, const ParticleInput& in, int N, int depth, 
 	LFMM_CUDA(ctx, cudaMemsetAsync(E.inner, 0, sizeof(double2) * lo * E.Nx2, s));
 	// upward
 	if (depth > 2)                         // no far pairs on levels 0 and 1
-		p2m_kernel<<<div_up(t.lsize[LL], WPB), WPB * 32, 0, s>>>(t, E, ctx.tables.d.knm);
+		if ((st = plain_p2m(ctx, t, N, E.outer))) return st;
 	// factored translations unless the per-pair rotations are asked for; the
 	// upward pass ends at level 2, the coarsest with far pairs
 	const bool rot = ctx.m2l_engine != 1;
@@ -550,7 +386,7 @@ int fmm3d_solve_device(Context& ctx, const ParticleInput& in, int N, int depth, 
 		}
 	}
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[4], s));
-	leaves_kernel<<<(unsigned)t.lsize[LL], LEAF_THREADS, 0, s>>>(t, E, ctx.tables.d.knm, pot, field);
+	if ((st = plain_leaves(ctx, t, N, depth > 2 ? E.inner : nullptr, pot, field))) return st;
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[5], s));
 	LFMM_CUDA(ctx, cudaGetLastError());
 	if (stats) {

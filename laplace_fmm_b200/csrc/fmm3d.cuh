@@ -39,6 +39,12 @@ int fmm3d_solve_scaled(Context& ctx, const ParticleInput& in, int N, int depth, 
 int fmm3d_scaled_on_tree(Context& ctx, const DevTree& t, int N, int precision, double* pot, double* field,
                          SolveStats* stats, const int* level_N = nullptr);
 
+// The plain form's leaves (uniform tree, unscaled expansions [cell][Nx2]): P2M
+// of every leaf, and the near field with (inner != nullptr) the local
+// expansions, written to pot and field in input order.
+int plain_p2m(Context& ctx, const DevTree& t, int N, double2* outer);
+int plain_leaves(Context& ctx, const DevTree& t, int N, const double2* inner, double* pot, double* field);
+
 // Dense FP64 M2L operators [343][MT][MT] for cell size h (h = 1: the
 // level-independent scaled operators), cached in the context.
 double* m2l_ops_fp64(Context& ctx, int N, double h);

@@ -283,6 +283,31 @@ int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, S
 
 } // namespace
 
+int plain_p2m(Context& ctx, const DevTree& t, int N, double2* outer)
+{
+	if (int st = upload_scaled_constants(ctx)) return st;
+	by_steps(N, [&](auto st_) {
+		p2m_plain_kernel<decltype(st_)::value>
+			<<<div_up(t.lsize[t.depth - 1], FWPB), FWPB * 32, 0, ctx.stream>>>(t, N, outer);
+	});
+	LFMM_CUDA(ctx, cudaGetLastError());
+	return OK;
+}
+
+int plain_leaves(Context& ctx, const DevTree& t, int N, const double2* inner, double* pot, double* field)
+{
+	if (int st = upload_scaled_constants(ctx)) return st;
+	const unsigned nl = (unsigned)t.lsize[t.depth - 1];
+	const dim3 grid(nl, std::min(64u, std::max(1u, 4u * (unsigned)ctx.num_sms / nl)));
+	const size_t smem = eval_smem<double>(1, N);
+	if (inner)
+		leaves_plain_kernel<true><<<grid, FWL * 32, smem, ctx.stream>>>(t, inner, N, pot, field);
+	else
+		leaves_plain_kernel<false><<<grid, FWL * 32, 0, ctx.stream>>>(t, inner, N, pot, field);
+	LFMM_CUDA(ctx, cudaGetLastError());
+	return OK;
+}
+
 float* m2l_ops_fp32(Context& ctx, int N)
 {
 	for (auto& e : ctx.opcache)
