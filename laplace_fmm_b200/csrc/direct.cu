@@ -114,8 +114,12 @@ __global__ void direct_reduce_kernel(size_t nt, int S, const double* __restrict_
 
 // Target i against the sources of its own segment [poff[seg[i]], poff[seg[i] + 1])
 // (the sampled checks of a batch of problems in one launch): one block per
-// target, the threads splitting the segment's sources, then a block
-// reduction in fixed order.  3D, 1/r as in the FAST sums.
+// DSEG targets, the threads splitting the segment's sources, then a block
+// reduction in fixed order; neighbouring targets of one segment share the
+// reads of its sources (the checks of 256 problems: 10.6 ms with one target per
+// block, 8.3 with 4, 10.4 with 8).  3D, 1/r as in the FAST sums.
+constexpr int DSEG = 4;
+
 __global__ void __launch_bounds__(DT) direct_segments_kernel(const double* __restrict__ src,
                                                              const double* __restrict__ q,
                                                              const uint32_t* __restrict__ poff,
@@ -123,33 +127,52 @@ __global__ void __launch_bounds__(DT) direct_segments_kernel(const double* __res
                                                              const double* __restrict__ tgt,
                                                              double* __restrict__ pot, double* __restrict__ fld)
 {
-	const size_t i = blockIdx.x;
-	if (i >= m) return;
-	const int k = seg[i];
-	const size_t lo = poff[k], hi = poff[k + 1];
-	const double xi = tgt[3 * i], yi = tgt[3 * i + 1], zi = tgt[3 * i + 2];
-	double v[4] = {0, 0, 0, 0};
-	for (size_t j = lo + threadIdx.x; j < hi; j += DT) {
-		const double dx = xi - src[3 * j], dy = yi - src[3 * j + 1], dz = zi - src[3 * j + 2];
-		const double inv = rsqrt_refined(fmax(dx * dx + dy * dy + dz * dz, FORCE_EPS2));
-		const double qr = q[j] * inv;
-		const double qr3 = qr * inv * inv;
-		v[0] += qr;
-		v[1] = fma(dx, qr3, v[1]); v[2] = fma(dy, qr3, v[2]); v[3] = fma(dz, qr3, v[3]);
-	}
-	__shared__ double red[DT / 32][4];
+	__shared__ double red[DT / 32][DSEG][4];
+	const size_t i0 = (size_t)blockIdx.x * DSEG, i1 = min(m, i0 + DSEG);
+	for (size_t a = i0; a < i1;) {             // runs of one segment
+		const int k = seg[a];
+		size_t b = a + 1;
+		while (b < i1 && seg[b] == k) ++b;
+		double x[DSEG][3], v[DSEG][4];
 #pragma unroll
-	for (int c = 0; c < 4; ++c) {
-		double x = v[c];
-		for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-		if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][c] = x;
-	}
-	__syncthreads();
-	if (threadIdx.x < 4) {
-		double x = 0.0;
-		for (int w = 0; w < DT / 32; ++w) x += red[w][threadIdx.x];
-		if (threadIdx.x == 0) pot[i] = x;
-		else fld[3 * i + threadIdx.x - 1] = x;
+		for (int u = 0; u < DSEG; ++u) {
+			const size_t i = min(a + u, b - 1);
+#pragma unroll
+			for (int c = 0; c < 3; ++c) x[u][c] = tgt[3 * i + c];
+			v[u][0] = v[u][1] = v[u][2] = v[u][3] = 0.0;
+		}
+		const size_t hi = poff[k + 1];
+		for (size_t j = poff[k] + threadIdx.x; j < hi; j += DT) {
+			const double sx = src[3 * j], sy = src[3 * j + 1], sz = src[3 * j + 2], sq = q[j];
+#pragma unroll
+			for (int u = 0; u < DSEG; ++u) {
+				if (a + u >= b) break;
+				const double dx = x[u][0] - sx, dy = x[u][1] - sy, dz = x[u][2] - sz;
+				const double inv = rsqrt_refined(fmax(dx * dx + dy * dy + dz * dz, FORCE_EPS2));
+				const double qr = sq * inv;
+				const double qr3 = qr * inv * inv;
+				v[u][0] += qr;
+				v[u][1] = fma(dx, qr3, v[u][1]); v[u][2] = fma(dy, qr3, v[u][2]); v[u][3] = fma(dz, qr3, v[u][3]);
+			}
+		}
+#pragma unroll
+		for (int u = 0; u < DSEG; ++u)
+#pragma unroll
+			for (int c = 0; c < 4; ++c) {
+				double y = v[u][c];
+				for (int o = 16; o; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+				if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][u][c] = y;
+			}
+		__syncthreads();
+		const int u = threadIdx.x >> 2, c = threadIdx.x & 3;
+		if (u < DSEG && a + u < b) {
+			double y = 0.0;
+			for (int w = 0; w < DT / 32; ++w) y += red[w][u][c];
+			if (c == 0) pot[a + u] = y;
+			else fld[3 * (a + u) + c - 1] = y;
+		}
+		__syncthreads();
+		a = b;
 	}
 }
 
@@ -159,7 +182,7 @@ int direct_segments_device(Context& ctx, const double* src, const double* q, con
                            const int32_t* seg, size_t m, const double* tgt, double* pot, double* fld)
 {
 	if (m == 0) return OK;
-	direct_segments_kernel<<<(unsigned)m, DT, 0, ctx.stream>>>(src, q, poff, seg, m, tgt, pot, fld);
+	direct_segments_kernel<<<div_up(m, DSEG), DT, 0, ctx.stream>>>(src, q, poff, seg, m, tgt, pot, fld);
 	LFMM_CUDA(ctx, cudaGetLastError());
 	return OK;
 }

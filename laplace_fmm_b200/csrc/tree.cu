@@ -85,32 +85,39 @@ __global__ void __launch_bounds__(BBOX_THREADS) bbox_partial_kernel(const Partic
 }
 
 // shift = min - 1e-7, scale = largest extent + 1e-6 (reference cpu/morton_tree.cpp:293-301)
-// One warp: lane l folds the partials l, l + 32, ..., then shuffles.
+// One block: thread k folds the partials k, k + 256, ..., then shuffles (one
+// warp, 32 dependent rounds of loads, took 12 us of every solve).
 template <int DIM>
-__global__ void bbox_final_kernel(const double* partial, int nb, double* geo)
+__global__ void __launch_bounds__(BBOX_THREADS) bbox_final_kernel(const double* partial, int nb, double* geo)
 {
-	const int lane = threadIdx.x;
-	if (lane >= 32) return;
 	double mn[DIM], mx[DIM];
 	for (int d = 0; d < DIM; ++d) { mn[d] = partial[d]; mx[d] = partial[DIM + d]; }
-	for (int b = lane; b < nb; b += 32)
+	for (int b = threadIdx.x; b < nb; b += BBOX_THREADS)
 		for (int d = 0; d < DIM; ++d) { mn[d] = fmin(mn[d], partial[b * 2 * DIM + d]); mx[d] = fmax(mx[d], partial[b * 2 * DIM + DIM + d]); }
 	for (int d = 0; d < DIM; ++d)
 		for (int o = 16; o > 0; o >>= 1) {
 			mn[d] = fmin(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
 			mx[d] = fmax(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
 		}
-	if (lane != 0) return;
+	__shared__ double s[BBOX_THREADS / 32][2 * DIM];
+	if ((threadIdx.x & 31) == 0)
+		for (int d = 0; d < DIM; ++d) { s[threadIdx.x >> 5][d] = mn[d]; s[threadIdx.x >> 5][DIM + d] = mx[d]; }
+	__syncthreads();
+	if (threadIdx.x != 0) return;
+	for (int k = 1; k < BBOX_THREADS / 32; ++k)
+		for (int d = 0; d < DIM; ++d) { mn[d] = fmin(mn[d], s[k][d]); mx[d] = fmax(mx[d], s[k][DIM + d]); }
 	double dw = mx[0] - mn[0];
 	for (int d = 1; d < DIM; ++d) dw = fmax(dw, mx[d] - mn[d]);
 	for (int d = 0; d < 3; ++d) geo[d] = d < DIM ? mn[d] - 1.e-7 : 0.0;
 	geo[3] = dw + 1.e-6;
 }
 
-// Forest: the bounding box of each problem, one block per problem, with the
-// same shift / scale rule.
+// Forest: the bounding box of each problem, one block per problem (the largest
+// sets the time: 1024 threads, 256 took 925 us for 262,144 particles), with
+// the same shift / scale rule.
+constexpr int SEG_THREADS = 1024;
 template <int DIM>
-__global__ void __launch_bounds__(BBOX_THREADS) bbox_segment_kernel(const ParticleInput in, double* geo)
+__global__ void __launch_bounds__(SEG_THREADS) bbox_segment_kernel(const ParticleInput in, double* geo)
 {
 	const uint32_t b = in.poff[blockIdx.x], e = in.poff[blockIdx.x + 1];
 	double mn[DIM], mx[DIM];
@@ -123,13 +130,13 @@ __global__ void __launch_bounds__(BBOX_THREADS) bbox_segment_kernel(const Partic
 			mn[d] = fmin(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
 			mx[d] = fmax(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
 		}
-	__shared__ double s[BBOX_THREADS / 32][2 * DIM];
+	__shared__ double s[SEG_THREADS / 32][2 * DIM];
 	const int w = threadIdx.x >> 5;
 	if ((threadIdx.x & 31) == 0)
 		for (int d = 0; d < DIM; ++d) { s[w][d] = mn[d]; s[w][DIM + d] = mx[d]; }
 	__syncthreads();
 	if (threadIdx.x == 0) {
-		for (int k = 1; k < BBOX_THREADS / 32; ++k)
+		for (int k = 1; k < SEG_THREADS / 32; ++k)
 			for (int d = 0; d < DIM; ++d) { s[0][d] = fmin(s[0][d], s[k][d]); s[0][DIM + d] = fmax(s[0][DIM + d], s[k][DIM + d]); }
 		double dw = s[0][DIM] - s[0][0];
 		for (int d = 1; d < DIM; ++d) dw = fmax(dw, s[0][DIM + d] - s[0][d]);
@@ -462,15 +469,15 @@ int tree_build(Context& ctx, const ParticleInput& in, int depth, DevTree& t, boo
 	LFMM_CUDA(ctx, cudaMemsetAsync(hist, 0, sizeof(unsigned) * (MAX_LEVELS + 2), s));
 	const unsigned TB = 256;
 	if (dim == 3 && nprob > 1) {
-		bbox_segment_kernel<3><<<nprob, BBOX_THREADS, 0, s>>>(in, t.geo);
+		bbox_segment_kernel<3><<<nprob, SEG_THREADS, 0, s>>>(in, t.geo);
 		codes_kernel<3><<<div_up(n, CODES_THREADS), CODES_THREADS, 0, s>>>(in, n, t.geo, depth, keys, vals);
 	} else if (dim == 3) {
 		bbox_partial_kernel<3><<<BBOX_BLOCKS, BBOX_THREADS, 0, s>>>(in, n, partial);
-		bbox_final_kernel<3><<<1, 32, 0, s>>>(partial, BBOX_BLOCKS, t.geo);
+		bbox_final_kernel<3><<<1, BBOX_THREADS, 0, s>>>(partial, BBOX_BLOCKS, t.geo);
 		codes_kernel<3><<<div_up(n, CODES_THREADS), CODES_THREADS, 0, s>>>(in, n, t.geo, depth, keys, vals);
 	} else {
 		bbox_partial_kernel<2><<<BBOX_BLOCKS, BBOX_THREADS, 0, s>>>(in, n, partial);
-		bbox_final_kernel<2><<<1, 32, 0, s>>>(partial, BBOX_BLOCKS, t.geo);
+		bbox_final_kernel<2><<<1, BBOX_THREADS, 0, s>>>(partial, BBOX_BLOCKS, t.geo);
 		codes_kernel<2><<<div_up(n, CODES_THREADS), CODES_THREADS, 0, s>>>(in, n, t.geo, depth, keys, vals);
 	}
 	int which = radix_sort_pairs(keys, vals, keys2, vals2, n, 0, dim * (depth - 1) + pbits, scratch, s);
