@@ -66,6 +66,10 @@ __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 // (-1)^n as a double
 __device__ __forceinline__ double dsgn(int n) { return (n & 1) ? -1.0 : 1.0; }
 
+// x >= 1e300, infinite, NaN or negative, from the high word: an integer
+// comparison, since the kernels that ask are bound by the FP64 pipe.
+__device__ __forceinline__ bool beyond_1e300(double x) { return (unsigned)__double2hiint(x) >= 0x7E37E43Cu; }
+
 // 1 / sqrt(x), x > 0: the hardware's FP64 reciprocal square root approximation
 // (rsqrt.approx.ftz.f64, no FP32 round trip; measured seed error 2^-20.1)
 // refined by one third-order step of the binomial series (1 - r)^(-1/2) =
@@ -74,7 +78,7 @@ __device__ __forceinline__ double dsgn(int n) { return (n & 1) ? -1.0 : 1.0; }
 // divide above 1e300.
 __device__ __forceinline__ double rsqrt_refined(double x)
 {
-	if (!(x < 1e300)) return 1.0 / sqrt(x);
+	if (beyond_1e300(x)) return 1.0 / sqrt(x);
 	double y;
 	asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
 	const double r = fma(-x * y, y, 1.0);
@@ -86,7 +90,7 @@ __device__ __forceinline__ double rsqrt_refined(double x)
 // below 2^-18 leaves e^3 < 2^-54).  The FP64 divide above 1e300.
 __device__ __forceinline__ double recip_refined(double x)
 {
-	if (!(x < 1e300)) return 1.0 / x;
+	if (beyond_1e300(x)) return 1.0 / x;
 	double y;
 	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
 	const double e = fma(-x, y, 1.0);

@@ -76,13 +76,58 @@ __device__ __forceinline__ double2 cpow_u(double2 b, int e)
 }
 __device__ __forceinline__ void coords2(uint64_t code, int* c) { c[0] = (int)compact2(code >> 1); c[1] = (int)compact2(code); }
 
-// a_k = -sum q (z - z0)^k / k, a_0 = sum q.  Lane k accumulates coefficient
-// k over the leaf's particles, staged 32 at a time.  Uniform tree: the leaves
-// of the last level; adaptive: every leaf, its sources [pbeg, send).
+// Power sums of sources, eight lanes per source and four sources per warp: lane
+// l of a group keeps sum q z^k for k = l, l + 8, l + 16, l + 24 (z^l from z, z^2
+// and z^4, then steps of z^8), about 37 FP64 operations per lane.  A lane per
+// coefficient that raised each source to its power took about 40 per source
+// and lane (P2M of 4.2M clustered particles at N = 21: 583 us).
+struct PowSums {
+	double2 a[4];
+	__device__ __forceinline__ void clear()
+	{
+#pragma unroll
+		for (int j = 0; j < 4; ++j) a[j] = make_double2(0.0, 0.0);
+	}
+	__device__ __forceinline__ void add(double2 z, double q, int N)
+	{
+		const int l = threadIdx.x & 7;
+		const double2 z2 = cmul(z, z), z4 = cmul(z2, z2), z8 = cmul(z4, z4);
+		double2 p = (l & 1) ? z : make_double2(1.0, 0.0);
+		if (l & 2) p = cmul(p, z2);
+		if (l & 4) p = cmul(p, z4);
+		p.x *= q; p.y *= q;
+#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			if (8 * j >= N) break;
+			a[j].x += p.x; a[j].y += p.y;
+			p = cmul(p, z8);
+		}
+	}
+	// the first cnt lanes' sources (the others: q = 0, z finite)
+	__device__ __forceinline__ void add32(double2 z, double q, int cnt, int N)
+	{
+		const int gr = (threadIdx.x & 31) >> 3;
+		for (int r = 0; r < cnt; r += 4)
+			add(make_double2(__shfl_sync(0xffffffffu, z.x, r + gr), __shfl_sync(0xffffffffu, z.y, r + gr)),
+			    __shfl_sync(0xffffffffu, q, r + gr), N);
+	}
+	// the four groups' sums, in every lane
+	__device__ __forceinline__ void reduce()
+	{
+#pragma unroll
+		for (int j = 0; j < 4; ++j)
+#pragma unroll
+			for (int o = 8; o < 32; o <<= 1) {
+				a[j].x += __shfl_xor_sync(0xffffffffu, a[j].x, o);
+				a[j].y += __shfl_xor_sync(0xffffffffu, a[j].y, o);
+			}
+	}
+};
+
+// a_k = -sum q (z - z0)^k / k, a_0 = sum q; warp per leaf.  Uniform tree: the
+// leaves of the last level; adaptive: every leaf, its sources [pbeg, send).
 __global__ void __launch_bounds__(WPB2 * 32) p2m2d_kernel(DevTree t, Exp2 E)
 {
-	__shared__ double2 sz[WPB2][32];
-	__shared__ double sq[WPB2][32];
 	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 	const size_t leaf = (size_t)blockIdx.x * WPB2 + w;
 	size_t g;
@@ -99,25 +144,22 @@ __global__ void __launch_bounds__(WPB2 * 32) p2m2d_kernel(DevTree t, Exp2 E)
 	}
 	const int N = E.N;
 	const double cx = t.cx[g], cy = t.cy[g];
-	double2 acc = make_double2(0.0, 0.0);
+	PowSums P;
+	P.clear();
 	for (uint32_t base = pb; base < pe; base += 32) {
-		const int cnt = (int)min(32u, pe - base);
-		__syncwarp();
-		if (lane < cnt) {
-			const uint32_t i = base + lane;
-			sq[w][lane] = t.q[i];
-			sz[w][lane] = make_double2(t.x[i] - cx, t.y[i] - cy);
-		}
-		__syncwarp();
-		if (lane < N)
-			for (int j = 0; j < cnt; ++j) {
-				const double2 p = cpow_u(sz[w][j], lane);
-				acc.x = fma(sq[w][j], p.x, acc.x); acc.y = fma(sq[w][j], p.y, acc.y);
-			}
+		const uint32_t i = base + lane;
+		double q = 0.0;
+		double2 z = make_double2(0.0, 0.0);
+		if (i < pe) { q = t.q[i]; z = make_double2(t.x[i] - cx, t.y[i] - cy); }
+		P.add32(z, q, (int)min(32u, pe - base), N);
 	}
-	if (lane < N) {
-		if (lane > 0) acc = make_double2(-acc.x / lane, -acc.y / lane);
-		E.outer[g * N + lane] = acc;
+	P.reduce();
+	if (lane < 8) {
+#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			const int k = lane + 8 * j;
+			if (k < N) E.outer[g * N + k] = k ? make_double2(-P.a[j].x / k, -P.a[j].y / k) : P.a[j];
+		}
 	}
 }
 
@@ -265,7 +307,10 @@ __global__ void __launch_bounds__(WPB2 * 32) l2l2d_add_kernel(DevTree t, Exp2 E,
 // Leaves: P2P over the close list (the leaf itself first) and L2P
 // (reference cpu/multipole.cpp:233-449).  One warp per work unit, a leaf's
 // targets in chunks of 32 (so a crowded leaf of a clustered set spreads over
-// many warps); a leaf of nt <= 16 targets is one unit whose warp runs TP = nt
+// many warps; bound by the FP64 pipe, about 24 operations per pair: 1/r^2 by
+// recip_refined instead of a division took the leaves of 4.2M clustered
+// particles from 3.75 to 3.59 ms, eight conflict-free copies of a 129-entry
+// table with one more term of the series back to 3.75); a leaf of nt <= 16 targets is one unit whose warp runs TP = nt
 // rounded up to a power of two targets at once and splits the sources into
 // 32 / TP phases, summed by shuffles at the end.
 constexpr int LW2 = 4;
@@ -360,7 +405,7 @@ __global__ void __launch_bounds__(LW2 * 32) leaves2d_kernel(DevTree t, Exp2 E, c
 					const double dx = xi - sx[w][k], dy = yi - sy[w][k];
 					const double r2 = fmax(dx * dx + dy * dy, FORCE_EPS2);
 					pot = fma(sq[w][k], log_table(r2, slog, ln2_hi, ln2_lo), pot);     // halved below
-					const double qr = sq[w][k] / r2;
+					const double qr = sq[w][k] * recip_refined(r2);
 					fr = fma(dx, qr, fr); fi = fma(-dy, qr, fi);
 				}
 			}
@@ -392,15 +437,13 @@ __global__ void __launch_bounds__(LW2 * 32) leaves2d_kernel(DevTree t, Exp2 E, c
 // P2L over the X list: cell B's Taylor series gains the log of every source
 // of a leaf C in X(B) (a monopole, so the series is exact in its terms):
 // b_0 += q conj(log(-d)), b_i += -q / (i d^i), d = z_j - c_B (the M2L rule of
-// down2d_kernel with a_0 = q and no other terms).  Warp per cell; sources
-// taken 16 at a time: lane j < 16 stages source j's log term and the powers
-// d^-1 .. d^-(N-1) (N - 1 products, once per source), then lane i sums
-// coefficient i over the 16 sources.
-constexpr int P2L_CHUNK = 16;
-
+// down2d_kernel with a_0 = q and no other terms).  Warp per cell; the sources
+// of 32 list entries as one sequence, 32 at a time: lane = source for the
+// logarithm, then the power sums of 1 / d.  (16 sources at a time, half the
+// lanes on the logarithms and the powers through shared memory, took 730 us on
+// the 4.2M clustered set.)
 __global__ void __launch_bounds__(WPB2 * 32) p2l2d_kernel(DevTree t, Exp2 E)
 {
-	__shared__ double2 spw[WPB2][P2L_CHUNK][MAXN2];   // [source][i]: q d^-i (i >= 1); [0]: q conj(log(-d))
 	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 	const size_t g = (size_t)blockIdx.x * WPB2 + w;
 	if (g >= t.ncells) return;
@@ -408,43 +451,52 @@ __global__ void __launch_bounds__(WPB2 * 32) p2l2d_kernel(DevTree t, Exp2 E)
 	if (xb == xe) return;
 	const int N = E.N;
 	const double cx = t.cx[g], cy = t.cy[g];
-	double2 acc = make_double2(0.0, 0.0);
-	const double inv_i = lane > 0 ? -1.0 / (double)lane : 0.0;
-	for (uint32_t e = xb; e < xe; ++e) {
-		const int32_t C = t.x_idx[e];
-		const uint32_t pb = t.pbeg[C], pe = t.send[C];
-		for (uint32_t base = pb; base < pe; base += P2L_CHUNK) {
-			const int cnt = (int)min((uint32_t)P2L_CHUNK, pe - base);
-			__syncwarp();
-			if (lane < cnt) {
-				const uint32_t i = base + lane;
-				const double qj = t.q[i];
-				const double dx = t.x[i] - cx, dy = t.y[i] - cy;
-				const double r2 = dx * dx + dy * dy;
-				spw[w][lane][0] = make_double2(qj * 0.5 * log(r2), -qj * atan2(-dy, -dx));
-				const double2 inv = make_double2(dx / r2, -dy / r2);
-				double2 p = make_double2(qj * inv.x, qj * inv.y);
-				for (int k = 1; k < N; ++k) {
-					spw[w][lane][k] = p;
-					p = cmul(p, inv);
-				}
+	PowSums P;
+	P.clear();
+	double2 lg = make_double2(0.0, 0.0);
+	for (uint32_t e0 = xb; e0 < xe; e0 += 32) {
+		uint32_t b = 0, n = 0;
+		if (e0 + lane < xe) {
+			const int32_t C = t.x_idx[e0 + lane];
+			b = t.pbeg[C]; n = t.send[C] - b;
+		}
+		uint32_t pre = n;                      // inclusive prefix sums of the entries' sources
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1) {
+			const uint32_t v = __shfl_up_sync(0xffffffffu, pre, o);
+			if (lane >= o) pre += v;
+		}
+		const uint32_t total = __shfl_sync(0xffffffffu, pre, 31), first = b - (pre - n);
+		for (uint32_t f0 = 0; f0 < total; f0 += 32) {
+			const uint32_t f = f0 + lane;
+			int k = 0;                         // the entry of source f: the prefixes <= f
+#pragma unroll
+			for (int o = 16; o > 0; o >>= 1)
+				if (__shfl_sync(0xffffffffu, pre, k + o - 1) <= f) k += o;
+			const uint32_t i = f + __shfl_sync(0xffffffffu, first, k & 31);
+			double q = 0.0;
+			double2 z = make_double2(0.0, 0.0);
+			if (f < total) {
+				q = t.q[i];
+				const double dx = t.x[i] - cx, dy = t.y[i] - cy, r2 = dx * dx + dy * dy;
+				z = make_double2(dx / r2, -dy / r2);
+				lg.x += q * 0.5 * log(r2); lg.y -= q * atan2(-dy, -dx);
 			}
-			__syncwarp();
-			if (lane < N) {
-				if (lane == 0)
-					for (int j = 0; j < cnt; ++j) { acc.x += spw[w][j][0].x; acc.y += spw[w][j][0].y; }
-				else
-					for (int j = 0; j < cnt; ++j) {
-						const double2 v = spw[w][j][lane];
-						acc.x = fma(inv_i, v.x, acc.x); acc.y = fma(inv_i, v.y, acc.y);
-					}
-			}
+			P.add32(z, q, (int)min(32u, total - f0), N);
 		}
 	}
-	if (lane < N) {
-		double2 b = E.inner[g * N + lane];
-		b.x += acc.x; b.y += acc.y;
-		E.inner[g * N + lane] = b;
+	P.reduce();
+	lg.x = warp_sum(lg.x); lg.y = warp_sum(lg.y);
+	if (lane < 8) {
+#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			const int k = lane + 8 * j;
+			if (k >= N) continue;
+			double2 v = E.inner[g * N + k];
+			if (k) { v.x -= P.a[j].x / k; v.y -= P.a[j].y / k; }
+			else { v.x += lg.x; v.y += lg.y; }
+			E.inner[g * N + k] = v;
+		}
 	}
 }
 
@@ -538,7 +590,7 @@ __global__ void __launch_bounds__(LW2 * 32) leaves2d_adaptive_kernel(DevTree t, 
 					const double dx = xi - sx[w][k], dy = yi - sy[w][k];
 					const double r2 = fmax(dx * dx + dy * dy, FORCE_EPS2);
 					pot = fma(sq[w][k], log_table(r2, slog, ln2_hi, ln2_lo), pot);     // halved below
-					const double qr = sq[w][k] / r2;
+					const double qr = sq[w][k] * recip_refined(r2);
 					fr = fma(dx, qr, fr); fi = fma(-dy, qr, fi);
 				}
 			}

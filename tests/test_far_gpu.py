@@ -1,6 +1,6 @@
 """Leaf kernels of the scaled form: chains of harmonics over eight lanes (P2M,
 P2L), evaluation with two or three targets per lane (M2P, L2P), short and long
-X / W lists; and of the plain form.  Orders at the edges of the chain kernels'
+X / W lists; of the plain form; and the 2D power sums.  Orders at the edges of the chain kernels'
 instances; split thresholds whose leaves fall on every pass size (up to 4, 8,
 12, 16, 24, 32, 48 targets and more than one pass); a narrow cluster beside a
 coarse background gives lists of 1 to hundreds of entries.
@@ -14,7 +14,7 @@ degree.  The mixed form must stay within its 1e-6 of the FP64 form."""
 import numpy as np
 import pytest
 
-from laplace_fmm_b200 import FastMultipole3d, InteractionType, compute_exact
+from laplace_fmm_b200 import FastMultipole, FastMultipole3d, InteractionType, compute_exact
 from laplace_fmm_b200.workloads import rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -57,3 +57,17 @@ def test_plain_leaves(ctx, oracle, N, n, depth):
     assert rel_l2(f.potentials, pot) < 1e-12
     if n > 1:
         assert rel_l2(f.forces, fld) < 1e-12
+
+
+@pytest.mark.parametrize("N", [1, 2, 8, 9, 16, 17, 25, 30])
+@pytest.mark.parametrize("n,depth", [(5, 3), (700, 4), (9001, 5)])
+def test_power_sums_2d(ctx, oracle, N, n, depth):
+    """The 2D power sums at the edges of their steps of eight orders, leaves of
+    a few to more than 32 sources, against the CPU restatement at the FP64
+    parity bar."""
+    g = np.random.Generator(np.random.PCG64(n + N))
+    src, q = g.random((n, 2)), g.uniform(0.1, 1, n)
+    f = FastMultipole((src, q), N=N, tree_depth=depth, ctx=ctx)
+    pot, fld = oracle.fmm2d(src, q, N=N, depth=depth)
+    assert rel_l2(f.potentials, pot) < 1e-12
+    assert rel_l2(np.stack([f.forces.real, f.forces.imag], 1), fld) < 1e-12
