@@ -287,9 +287,9 @@ def launches_per_solve(depth, dim, radix_passes, adaptive, precision, learned=Fa
     from the launch sites; the learned solve adds its features (far strength
     per level, accumulation per level, leaf features), the network, the
     prediction sums, the sampled direct sum (split kernel and reduction) and
-    the RMS and error sums.  An ncu launch list of the 16.8M-particle learned
-    solve shows 277 launches per solve: these 276 and the statistics pass of
-    a timing context."""
+    the RMS and error sums.  A trace of the 16.8M-particle learned solve shows
+    294 kernels per solve; this count of 283 leaves out the leaf-size
+    candidates' counts and the autotuned split reductions."""
     extra = (1 + (depth - 2) + (depth - 1) + 1 + 1 + 1 + 2 + 1 + 1) if learned else 0
     scan = 3
     tree = 2 + 1 + radix_passes * (1 + scan + 1) + 1 + 1 + scan + 1 + 1
@@ -297,12 +297,14 @@ def launches_per_solve(depth, dim, radix_passes, adaptive, precision, learned=Fa
     lists = depth - 1
     if adaptive or precision != "fp64":
         tree += depth + depth * (1 + scan) + depth + 1 + scan + 1 + 1 + lists + 2 + 2 + 3 * scan
-        # plan (class count, scatter, slot table) + GEMM per level; split
-        # reductions and FP64 converts on the coarse levels 2-3
-        m2l = max(0, depth - 2) * (3 + 1) + 2 + 2 * 2
-        m2m = (depth - 1) * (2 if precision == "mixed" else 1)  # mixed: plan + tensor-core GEMM per level
-        leaves = 2 if precision == "mixed" else 1               # FP32: near field, then the expansions
-        fmm = 1 + 1 + m2m + m2l + 1 + max(0, depth - 3) + leaves
+        # plan (class count, scatter, slot table) + translation per level,
+        # split reductions on levels 2-3, the mixed form's source staging
+        # (largest magnitude, split) on the finer ones
+        m2l = max(0, depth - 2) * (3 + 1) + 2 + (2 * max(0, depth - 4) if precision == "mixed" else 0)
+        m2m = 2 * max(0, depth - 3)                # plan + translation, levels depth-2 .. 2
+        # P2M, axial tables; P2L: list selection, short and long lists; L2L;
+        # near field, expansions of the leaves with short and with long lists
+        fmm = 1 + 1 + m2m + m2l + 3 + max(0, depth - 3) + 3
         return (tree, fmm) if parts else tree + fmm + extra
     if adaptive and dim == 2:
         tree += depth + depth * (1 + scan) + depth + 1 + scan + 1 + 1 + lists + 2 + 2 + 3 * scan
@@ -315,7 +317,8 @@ def launches_per_solve(depth, dim, radix_passes, adaptive, precision, learned=Fa
         return (tree, fmm) if parts else tree + fmm
     tree += lists
     if dim == 3:
-        fmm = 1 + (depth - 1) + max(0, depth - 2) * 5 + max(0, depth - 3) + 1
+        # P2M, axial tables, M2M (plan + translation), M2L, L2L, leaves
+        fmm = 1 + 1 + 2 * max(0, depth - 3) + max(0, depth - 2) * 5 + max(0, depth - 3) + 1
     else:
         # per level 2..depth-1: class count, scatter, slot table, Hankel M2L,
         # and a split reduction on the levels too small to fill the GPU

@@ -98,6 +98,30 @@ __global__ void __launch_bounds__(SCAN_BLOCK) scan_apply_kernel(const uint32_t* 
 	}
 }
 
+// Few elements: one tile of one block, one launch of 3-4 us instead of three of
+// 2 (two tiles take 12).
+constexpr int SMALL_BLOCK = 1024, SMALL_ITEMS = 8;
+constexpr size_t SCAN_SMALL = SMALL_BLOCK * SMALL_ITEMS;
+
+__global__ void __launch_bounds__(SMALL_BLOCK) scan_small_kernel(const uint32_t* in, uint32_t* out, size_t n,
+                                                                uint32_t* total)
+{
+	__shared__ uint32_t warp_tot[33];
+	const size_t base = (size_t)threadIdx.x * SMALL_ITEMS;
+	uint32_t v[SMALL_ITEMS];
+	uint32_t s = 0;
+#pragma unroll
+	for (int i = 0; i < SMALL_ITEMS; ++i) { v[i] = base + i < n ? in[base + i] : 0u; s += v[i]; }
+	uint32_t run;
+	const uint32_t tot = block_exclusive_scan<SMALL_BLOCK>(s, run, warp_tot);
+#pragma unroll
+	for (int i = 0; i < SMALL_ITEMS; ++i) {
+		if (base + i < n) out[base + i] = run;
+		run += v[i];
+	}
+	if (threadIdx.x == 0 && total) *total = tot;
+}
+
 // ---------------------------------------------------------------- radix
 constexpr int RADIX_BLOCK = 256;
 constexpr int RADIX_ROUNDS = 16;
@@ -179,6 +203,10 @@ void scan_exclusive_u32(const uint32_t* in, uint32_t* out, size_t n, uint32_t* t
 {
 	if (n == 0) {
 		if (total) cudaMemsetAsync(total, 0, sizeof(uint32_t), s);
+		return;
+	}
+	if (n <= SCAN_SMALL) {
+		scan_small_kernel<<<1, SMALL_BLOCK, 0, s>>>(in, out, n, total);
 		return;
 	}
 	size_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;

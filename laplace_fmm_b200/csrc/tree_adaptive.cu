@@ -152,8 +152,102 @@ __global__ void source_ranges_kernel(DevTree a)
 }
 
 // U and W lists of one leaf (pass 0: count, pass 1: fill at the offsets).
+struct UWCount { uint32_t u = 0, w = 0; };
+
+// The U and W entries of leaf B (level L, coords me) under its colleague C, in
+// the walk's order; written to u and w unless null.
+template <int DIM>
+__device__ UWCount uw_walk(const DevTree& a, int L, const int* me, int32_t C, int32_t* __restrict__ u,
+                           int32_t* __restrict__ w, unsigned* flags)
+{
+	UWCount n;
+	if (a.is_leaf[C]) {
+		if (u) u[0] = C;
+		n.u = 1;
+		return n;
+	}
+	int32_t stack[STACK];
+	int sp = 0;
+	for (uint32_t k = a.beg[C]; k < a.end[C]; ++k) stack[sp++] = (int32_t)(a.loff[L + 1] + k);
+	while (sp > 0) {
+		const int32_t D = stack[--sp];
+		const int ld = a.lev[D];
+		int d[3];
+		coords<DIM>(a.code[D], d);
+		if (touch<DIM>(L, me, ld, d)) {
+			if (a.is_leaf[D]) {
+				if (u) u[n.u] = D;
+				n.u++;
+			} else {
+				for (uint32_t k = a.beg[D]; k < a.end[D]; ++k) {
+					if (sp < STACK) stack[sp++] = (int32_t)(a.loff[ld + 1] + k);
+					else atomicOr(flags, DEV_ERR_LIST_OVERFLOW);
+				}
+			}
+		} else {
+			if (w) w[n.w] = D;
+			n.w++;
+		}
+	}
+	return n;
+}
+
+// A warp per leaf: lane e walks below the leaf's e-th colleague, then the lanes
+// test the colleagues of each ancestor; prefix sums over the lanes keep the
+// order of the colleagues.  Pass 0 counts, pass 1 writes.  (A thread per leaf:
+// 127 us a pass for 562 leaves, 180 for 15,227, one chain of dependent loads.)
 template <int DIM>
 __global__ void uw_kernel(DevTree a, int pass, uint32_t* __restrict__ ucnt, uint32_t* __restrict__ wcnt, unsigned* flags)
+{
+	const size_t li = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+	const int lane = threadIdx.x & 31;
+	if (li >= a.nleaves) return;
+	const int32_t g = a.leaves[li];
+	const int L = a.lev[g];
+	int me[3];
+	coords<DIM>(a.code[g], me);
+	const int nc = a.close_cnt[g];
+	const int32_t C = lane < nc ? (int32_t)(a.loff[L] + a.close_idx[(size_t)g * a.close_stride + lane]) : -1;
+	UWCount n;
+	if (C >= 0) n = uw_walk<DIM>(a, L, me, C, nullptr, nullptr, flags);
+	__syncwarp();
+	uint32_t iu = n.u, iw = n.w;               // inclusive prefix sums
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const uint32_t vu = __shfl_up_sync(0xffffffffu, iu, o), vw = __shfl_up_sync(0xffffffffu, iw, o);
+		if (lane >= o) { iu += vu; iw += vw; }
+	}
+	uint32_t nu = __shfl_sync(0xffffffffu, iu, 31);
+	const uint32_t nw = __shfl_sync(0xffffffffu, iw, 31);
+	const uint32_t ub = pass ? a.u_off[li] : 0, wb = pass ? a.w_off[li] : 0;
+	if (pass && C >= 0)
+		uw_walk<DIM>(a, L, me, C, a.u_idx + ub + (iu - n.u), a.w_idx + wb + (iw - n.w), flags);
+	__syncwarp();
+	// coarser adjacent leaves: leaf colleagues of the ancestors that touch B
+	int32_t A = g;
+	for (int l = L - 1; l >= 1; --l) {
+		A = (int32_t)(a.loff[l] + a.parent[A]);
+		int32_t D = -1;
+		if (lane < a.close_cnt[A]) {
+			D = (int32_t)(a.loff[l] + a.close_idx[(size_t)A * a.close_stride + lane]);
+			int c[3];
+			if (!a.is_leaf[D]) D = -1;
+			else {
+				coords<DIM>(a.code[D], c);
+				if (!touch<DIM>(l, c, L, me)) D = -1;
+			}
+		}
+		const uint32_t on = __ballot_sync(0xffffffffu, D >= 0);
+		if (pass && D >= 0) a.u_idx[ub + nu + __popc(on & ((1u << lane) - 1))] = D;
+		nu += __popc(on);
+	}
+	if (!pass && lane == 0) { ucnt[li] = nu; wcnt[li] = nw; }
+}
+
+// The same with a thread per leaf, for trees with leaves enough to hide its
+// dependent loads.
+template <int DIM>
+__global__ void uw_many_kernel(DevTree a, int pass, uint32_t* __restrict__ ucnt, uint32_t* __restrict__ wcnt, unsigned* flags)
 {
 	size_t li = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
 	if (li >= a.nleaves) return;
@@ -219,6 +313,19 @@ __global__ void uw_kernel(DevTree a, int pass, uint32_t* __restrict__ ucnt, uint
 		}
 	}
 	if (!pass) { ucnt[li] = nu; wcnt[li] = nw; }
+}
+
+// The line between them (B200, both passes): 3D 99 us a warp per leaf against
+// 207 a thread per leaf at 57,008 leaves, slower at 514,046; 2D (eight
+// colleagues) 537 against 82 on the 4.2M clustered set.
+template <int DIM> constexpr size_t uw_many() { return DIM == 3 ? 262144 : 16384; }
+
+template <int DIM>
+void launch_uw(const DevTree& a, int pass, uint32_t* ucnt, uint32_t* wcnt, unsigned* flags, cudaStream_t s)
+{
+	const size_t nl = a.nleaves;
+	if (nl > uw_many<DIM>()) uw_many_kernel<DIM><<<div_up(nl, 128), 128, 0, s>>>(a, pass, ucnt, wcnt, flags);
+	else uw_kernel<DIM><<<div_up(nl, 4), 128, 0, s>>>(a, pass, ucnt, wcnt, flags);
 }
 
 // X list of one cell: leaf colleagues C of an ancestor, touching parent(B)
@@ -478,10 +585,10 @@ int tree_build_adaptive(Context& ctx, const ParticleInput& in, int depth, int ma
 	uint32_t* tots = take<uint32_t>(ctx, 4);
 	if (!ucnt || !wcnt || !xcnt || !tots) { ctx.last_error = "adaptive tree: allocation failed"; return ERR_OOM; }
 	if (dim == 3) {
-		uw_kernel<3><<<div_up(nl, 128), 128, 0, s>>>(a, 0, ucnt, wcnt, ctx.dev_flags);
+		launch_uw<3>(a, 0, ucnt, wcnt, ctx.dev_flags, s);
 		x_kernel<3><<<div_up(C, 128), 128, 0, s>>>(a, 0, xcnt);
 	} else {
-		uw_kernel<2><<<div_up(nl, 128), 128, 0, s>>>(a, 0, ucnt, wcnt, ctx.dev_flags);
+		launch_uw<2>(a, 0, ucnt, wcnt, ctx.dev_flags, s);
 		x_kernel<2><<<div_up(C, 128), 128, 0, s>>>(a, 0, xcnt);
 	}
 	scan_exclusive_u32(ucnt, a.u_off, nl, a.u_off + nl, scr, s);
@@ -499,10 +606,10 @@ int tree_build_adaptive(Context& ctx, const ParticleInput& in, int depth, int ma
 	a.x_idx = take<int32_t>(ctx, a.n_x);
 	if (!a.u_idx || !a.w_idx || !a.x_idx) { ctx.last_error = "adaptive tree: allocation failed"; return ERR_OOM; }
 	if (dim == 3) {
-		uw_kernel<3><<<div_up(nl, 128), 128, 0, s>>>(a, 1, ucnt, wcnt, ctx.dev_flags);
+		launch_uw<3>(a, 1, ucnt, wcnt, ctx.dev_flags, s);
 		x_kernel<3><<<div_up(C, 128), 128, 0, s>>>(a, 1, xcnt);
 	} else {
-		uw_kernel<2><<<div_up(nl, 128), 128, 0, s>>>(a, 1, ucnt, wcnt, ctx.dev_flags);
+		launch_uw<2>(a, 1, ucnt, wcnt, ctx.dev_flags, s);
 		x_kernel<2><<<div_up(C, 128), 128, 0, s>>>(a, 1, xcnt);
 	}
 	LFMM_CUDA(ctx, cudaGetLastError());
