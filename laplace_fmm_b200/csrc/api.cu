@@ -11,6 +11,8 @@
 #include <new>
 #include <algorithm>
 #include <cstdlib>
+#include <mutex>
+#include <set>
 
 struct lfmm_ctx {
 	lfmm::Context c;
@@ -70,6 +72,19 @@ int cuda_fail(Context& ctx, cudaError_t e, const char* where)
 {
 	ctx.last_error = std::string("CUDA error ") + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ") at " + where;
 	return ERR_CUDA;
+}
+
+cudaError_t smem_limit(int device, const void* kernel, size_t bytes, bool max_shared)
+{
+	static std::mutex mu;
+	static std::set<std::pair<int, const void*>> set;
+	std::lock_guard<std::mutex> lock(mu);
+	if (set.count({device, kernel})) return cudaSuccess;
+	cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+	if (e == cudaSuccess && max_shared)
+		e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+	if (e == cudaSuccess) set.insert({device, kernel});
+	return e;
 }
 
 Context& ctx_of(lfmm_ctx* c) { return c->c; }

@@ -132,6 +132,15 @@ inline void opcache_make_room(Context& ctx)
 int tables_build(Context& ctx);
 void tables_free(Tables& t);
 
+// Let `kernel` be launched with up to `bytes` of dynamic shared memory (and,
+// with max_shared, prefer shared memory to L1).  The limit belongs to the
+// kernel in its device's primary context, which every solver context and host
+// thread shares, and a launch above it fails; so it is set once per device, to
+// the most that any launch of the kernel asks for, and never lowered (set to
+// each solve's own size before each launch, a second thread at a lower order
+// made the first one's launch fail; the two calls also took about 1 us).
+cudaError_t smem_limit(int device, const void* kernel, size_t bytes, bool max_shared = false);
+
 // set last_error from a CUDA error; returns ERR_CUDA
 int cuda_fail(Context& ctx, cudaError_t e, const char* where);
 

@@ -270,8 +270,8 @@ int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, S
 	else
 		p2p_f64_kernel<LWP><<<resident, LWP * 32, 0, s>>>(t, pot, field, next);
 	const size_t sm_e = eval_smem<real>(FWPB, N), sm_l = eval_smem<real>(FWL, N);
-	LFMM_CUDA(ctx, cudaFuncSetAttribute(eval_scaled_kernel<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_e));
-	LFMM_CUDA(ctx, cudaFuncSetAttribute(eval_long_kernel<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_l));
+	LFMM_CUDA(ctx, smem_limit(ctx.device, reinterpret_cast<const void*>(eval_scaled_kernel<real>), eval_smem<real>(FWPB, MAXN3)));
+	LFMM_CUDA(ctx, smem_limit(ctx.device, reinterpret_cast<const void*>(eval_long_kernel<real>), eval_smem<real>(FWL, MAXN3)));
 	eval_scaled_kernel<real><<<resident, FWPB * 32, sm_e, s>>>(t, outer, inner, N, pot, field, next + 1, longs);
 	if (t.n_w > FAR_SHORT)
 		eval_long_kernel<real><<<2 * ctx.num_sms, FWL * 32, sm_l, s>>>(t, outer, inner, N, pot, field, next + 2, longs);

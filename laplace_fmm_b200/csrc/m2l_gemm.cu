@@ -680,7 +680,7 @@ int m2l_hankel2d(Context& ctx, const M2LPlan& plan, const double2* tab, const do
 	const int MTL = (N + 7) / 8;           // row tiles of 8
 	const size_t smem = hankel_smem(N);
 	auto go = [&](auto kern) -> cudaError_t {
-		cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+		const cudaError_t e = smem_limit(ctx.device, reinterpret_cast<const void*>(kern), hankel_smem(8 * MTL));
 		if (e != cudaSuccess) return e;
 		kern<<<grid, 128, smem, s>>>(tab, mult, loc, plan.vtab, plan.order, plan.oct_count, N, part, plan.cells);
 		return cudaGetLastError();

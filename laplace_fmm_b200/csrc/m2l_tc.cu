@@ -1032,10 +1032,10 @@ int launch_tc(Context& ctx, const M2LPlan& plan, const uint4* ops, const float* 
               float t_inv)
 {
 	using C = TcCfg<NC, NA, !TMA, F16>;
-	LFMM_CUDA(ctx, cudaFuncSetAttribute(m2l_tc_kernel<NC, NA, M2L_SLOTS, TC_M2L, true, F16, TMA>,
-	                                    cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-	LFMM_CUDA(ctx, cudaFuncSetAttribute(m2l_tc_kernel<NC, NA, M2L_SLOTS, TC_M2L, false, F16, TMA>,
-	                                    cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+	auto *pers_k = m2l_tc_kernel<NC, NA, M2L_SLOTS, TC_M2L, true, F16, TMA>,
+	     *item_k = m2l_tc_kernel<NC, NA, M2L_SLOTS, TC_M2L, false, F16, TMA>;
+	LFMM_CUDA(ctx, smem_limit(ctx.device, reinterpret_cast<const void*>(pers_k), C::SMEM));
+	LFMM_CUDA(ctx, smem_limit(ctx.device, reinterpret_cast<const void*>(item_k), C::SMEM));
 	unsigned* bmax = nullptr;
 	uint4 *shi = nullptr, *slo = nullptr;
 	CUtensorMap maps[2];
@@ -1119,8 +1119,8 @@ template <int NC, int NA>
 int launch_m2m_tc(Context& ctx, const M2LPlan& plan, const uint4* ops, const float* src, float* dst, int R,
                   size_t src_cells)
 {
-	LFMM_CUDA(ctx, cudaFuncSetAttribute(m2l_tc_kernel<NC, NA, 8, TC_M2M, false, false, false>,
-	                                    cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<NC, NA>::SMEM));
+	auto* kern = m2l_tc_kernel<NC, NA, 8, TC_M2M, false, false, false>;
+	LFMM_CUDA(ctx, smem_limit(ctx.device, reinterpret_cast<const void*>(kern), TcCfg<NC, NA>::SMEM));
 	return run_tc<NC, NA, 8, TC_M2M>(ctx, plan, ops, src, dst, R, 1, nullptr, false, src_cells, 0, false);
 }
 

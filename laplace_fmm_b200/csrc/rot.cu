@@ -98,6 +98,30 @@ inline int rot_raw_ld(int N) { return (N * (N + 1) / 2 + 3) / 8 * 8 + 4; }   // 
 inline size_t rot_planes(int N) { return sizeof(double) * 2 * (size_t)rot_rows(N) * RLD; }
 inline size_t rot_raw(int N, size_t elem) { return elem * (size_t)RT * rot_raw_ld(N); }
 
+// Dynamic shared memory of order N; apart: the raw gather has a place of its
+// own beside X and Y where that leaves room for the blocks an SM holds (two up
+// to N = 12), else it lies in Y: apart, the next slot's sources arrive during
+// all three products instead of the last one.
+size_t rot_smem(int N, size_t elem, bool& apart)
+{
+	const size_t room = N <= 12 ? (size_t)101 << 10 : (size_t)206 << 10;
+	const size_t planes = rot_planes(N), raw = rot_raw(N, elem);
+	apart = 2 * planes + raw <= room;
+	return apart ? 2 * planes + raw : planes + std::max(planes, raw);
+}
+
+// Orders that share a kernel instance: the largest of N's.
+constexpr int rot_last(int N) { return N <= 8 ? 8 : N <= 12 ? 12 : N <= 16 ? 16 : MAXN3; }
+
+// The most shared memory that a launch of N's instance asks for.
+size_t rot_smem_limit(int N, size_t elem)
+{
+	size_t most = 0;
+	bool apart;
+	for (int n = rot_last(N); n > 0 && rot_last(n) == rot_last(N); --n) most = std::max(most, rot_smem(n, elem, apart));
+	return most;
+}
+
 // Block of 8 or 16 warps per (class, tile of at most 32 targets) and slot
 // range.  Per
 // non-empty slot, the sources present are gathered into consecutive columns
@@ -545,19 +569,12 @@ int rot_translate(Context& ctx, RotMode mode, const M2LPlan& plan, const real* s
 	const int nw = N <= 12 ? 8 : 16;
 	RotJobs J;
 	rot_jobs(N, nw, J);
-	// the raw gather beside X and Y where that leaves room for the blocks an SM
-	// holds (two up to N = 12), else in Y: the next slot's sources then arrive
-	// during all three products instead of the last one
-	const size_t room = N <= 12 ? (size_t)101 << 10 : (size_t)206 << 10;
-	const size_t planes = rot_planes(N), rawb = rot_raw(N, sizeof(v2));
-	const bool apart = 2 * planes + rawb <= room;
-	const size_t smem = apart ? 2 * planes + rawb : planes + std::max(planes, rawb);
+	bool apart;
+	const size_t smem = rot_smem(N, sizeof(v2), apart), limit = rot_smem_limit(N, sizeof(v2));
 	cudaStream_t s = ctx.stream;
 	const DevTables& T = ctx.tables.d;
 	auto go = [&](auto kern) -> cudaError_t {
-		cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-		if (e == cudaSuccess)
-			e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+		const cudaError_t e = smem_limit(ctx.device, reinterpret_cast<const void*>(kern), limit, true);
 		if (e != cudaSuccess) return e;
 		kern<<<dim3(tiles, S), nw * 32, smem, s>>>(reinterpret_cast<const v2*>(src), reinterpret_cast<v2*>(dst), plan.vtab,
 		                                           plan.order, plan.oct_count, N, T.rotf, T.emat, T.dirinfo, axial, J, apart, tile,
