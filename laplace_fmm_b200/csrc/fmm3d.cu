@@ -365,9 +365,15 @@ int fmm3d_solve_device(Context& ctx, const ParticleInput& in, int N, int depth, 
 	for (int L = 2; L < depth; ++L) {
 		if (rot) {
 			if ((st = m2l_plan_build(ctx, t, L, plans[L]))) return st;
-			if ((st = rot_translate<double>(ctx, ROT_M2L, plans[L], flat(E.outer, L), flat(E.inner, L), N,
-			                                rot_axial_level(ax, N, L))))
-				return st;
+			if (m2l_dense64(N, t.lsize[L])) {
+				const double* ops = m2l_ops_fp64(ctx, N, t.geo_host[3] / (double)(1ull << L));
+				if (!ops) return ERR_OOM;
+				st = m2l_gemm64(ctx, plans[L], ops, flat(E.outer, L), flat(E.inner, L), N);
+			} else {
+				st = rot_translate<double>(ctx, ROT_M2L, plans[L], flat(E.outer, L), flat(E.inner, L), N,
+				                           rot_axial_level(ax, N, L));
+			}
+			if (st) return st;
 		} else {
 			m2l_kernel<<<div_up(t.lsize[L], WPB), WPB * 32, 0, s>>>(t, E, L, ctx.tables.d, ctx.dev_flags);
 		}

@@ -152,6 +152,28 @@ void by_steps(int N, F go)
 	else go(std::integral_constant<int, 23>());
 }
 
+// The dense FP64 M2L of a level (m2l_dense64); FP32 expansions are widened
+// into scratch and rounded back.
+template <typename real>
+int dense64(Context& ctx, const M2LPlan& plan, const real* mult, real* loc, int N)
+{
+	const double* ops = m2l_ops_fp64(ctx, N, 1.0);
+	if (!ops) return ERR_OOM;
+	if constexpr (sizeof(real) == sizeof(double)) {
+		return m2l_gemm64(ctx, plan, ops, mult, loc, N);
+	} else {
+		const size_t n = plan.cells * (size_t)N * (N + 1);
+		double* m = static_cast<double*>(ctx.arena.take(sizeof(double) * n));
+		double* l = static_cast<double*>(ctx.arena.take(sizeof(double) * n));
+		if (!m || !l) { ctx.last_error = "scaled solve: allocation failed"; return ERR_OOM; }
+		convert_kernel<<<div_up(n, 256), 256, 0, ctx.stream>>>(mult, m, n);
+		if (int st = m2l_gemm64(ctx, plan, ops, m, l, N)) return st;
+		convert_kernel<<<div_up(n, 256), 256, 0, ctx.stream>>>(l, loc, n);
+		LFMM_CUDA(ctx, cudaGetLastError());
+		return OK;
+	}
+}
+
 template <typename real>
 int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, SolveStats* stats,
             const int* level_N)
@@ -217,7 +239,11 @@ int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, S
 			// a level's own source order (level_N) is the tensor-core engine's
 			const bool own_n = level_N && level_N[L] > 0 && level_N[L] < N;
 			if (!coarse64 || L <= 3 || (tc && t.lsize[L] <= ROT_M2L_CELLS && !own_n)) {
-				if ((st = rot_translate<real>(ctx, ROT_M2L, plan, mL, lL, N, ax))) return st;
+				if (m2l_dense64(N, t.lsize[L])) {
+					if ((st = dense64<real>(ctx, plan, mL, lL, N))) return st;
+				} else if ((st = rot_translate<real>(ctx, ROT_M2L, plan, mL, lL, N, ax))) {
+					return st;
+				}
 			} else if (tc) {
 				// tcgen05 hi/lo GEMM on the FP32 levels (FP16 or TF32 operands)
 				float t_inv = 1.f;
@@ -319,7 +345,7 @@ float* m2l_ops_fp32(Context& ctx, int N)
 	OpCacheEntry e;
 	e.N = N; e.prec = 1; e.h = 1.0; e.bytes = cnt * sizeof(float); e.stamp = ++ctx.opcache_clock;
 	if (cudaMalloc(&e.ptr, e.bytes) != cudaSuccess) { cudaGetLastError(); ctx.last_error = "m2l operators: out of memory"; return nullptr; }
-	convert_back_kernel<float><<<div_up(cnt, 256), 256, 0, ctx.stream>>>(d, static_cast<float*>(e.ptr), cnt);
+	convert_kernel<<<div_up(cnt, 256), 256, 0, ctx.stream>>>(d, static_cast<float*>(e.ptr), cnt);
 	ctx.opcache.push_back(e);
 	return static_cast<float*>(e.ptr);
 }

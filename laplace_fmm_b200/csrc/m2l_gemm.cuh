@@ -43,6 +43,17 @@ int m2l_plan_build(Context& ctx, const DevTree& t, int L, M2LPlan& plan);
 // (FP32, partial sums carried in FP64).  ops: [343][MT][MT].
 int m2l_gemm(Context& ctx, const M2LPlan& plan, const float* ops, const float* mult, float* loc, int N);
 
+// The same in FP64 on the FP64 tensor cores (ops: m2l_ops_fp64), for the levels
+// whose order is too low for the factored translations (rot.cuh), whose time is
+// barriers and latencies of a slot.  Uniform levels on B200, dense against
+// factored, us: N = 2 27 / 34 at 512 cells, 60 / 256 at 4,096, 2637 / 14029 at
+// 262,144; N = 5 48 / 39, 127 / 315, 6538 / 17808; N = 6 86 / 44, 220 / 351,
+// 11075 / 19724; N = 7 113 / 44, 296 / 369, 15105 / 21256; N = 8 169 / 49, 673 /
+// 405, 37275 / 23361.  Operators of a new cell size: 6-46 us.
+constexpr int M2L64_ORDER = 7, M2L64_ROWS = 64;      // highest order, its operator rows
+inline bool m2l_dense64(int N, size_t cells) { return N <= 5 ? cells > 512 : N <= M2L64_ORDER && cells > 2048; }
+int m2l_gemm64(Context& ctx, const M2LPlan& plan, const double* ops, const double* mult, double* loc, int N);
+
 // 2D (FP64, expansions [cell][N] complex): the quadrant classes' 27 far
 // slots, the dense operators [49][MT][MT] (MT = 2N rounded up to 16) of cell
 // size h, and the GEMM.

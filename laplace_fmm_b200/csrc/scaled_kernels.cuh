@@ -121,11 +121,11 @@ __device__ inline void translate_scaled(const double2* __restrict__ src, int dir
 template <typename real> __device__ __forceinline__ real rsq(real x);
 template <> __device__ __forceinline__ float rsq<float>(float x) { return rsqrtf(x); }
 template <> __device__ __forceinline__ double rsq<double>(double x) { return rsqrt(x); }
-template <typename real>
-__global__ void convert_back_kernel(const double* __restrict__ in, real* __restrict__ out, size_t n)
+template <typename from, typename to>
+__global__ void convert_kernel(const from* __restrict__ in, to* __restrict__ out, size_t n)
 {
 	size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i < n) out[i] = (real)in[i];
+	if (i < n) out[i] = (to)in[i];
 }
 
 // FP32 near field on its own (few registers, high occupancy): one warp per

@@ -9,7 +9,7 @@ import os
 import numpy as np
 import pytest
 
-from laplace_fmm_b200 import Context, FastMultipole3d
+from laplace_fmm_b200 import Context, FastMultipole3d, solve_batch
 from laplace_fmm_b200.workloads import rel_l2, uniform3d
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +65,32 @@ def test_scaled_translations_match_rotations(ctx, rotation, N, depth):
     tol = 5e-12 + 2 * N * 1e-12 * m
     assert rel_l2(a.potentials - q * 1e4, b.potentials - q * 1e4) < tol
     assert rel_l2(a.forces, b.forces) < tol
+
+
+# the low orders' dense FP64 M2L (levels above 512 or 2,048 cells) and the
+# factored one below the line, at the orders where the operators' row tiles
+# change; the same bar as above
+@pytest.mark.parametrize("N", [1, 3, 5, 6, 7, 8])
+@pytest.mark.parametrize("n,depth,nt", [(20000, 5, 0), (40000, 5, 3001)])
+def test_low_orders_match_rotations(ctx, rotation, N, n, depth, nt):
+    src, q = uniform3d(n, seed=50 + N)
+    args = ((src, q),) if nt == 0 else ((src, q), uniform3d(nt, seed=8)[0])
+    a = FastMultipole3d(*args, N=N, tree_depth=depth, ctx=ctx)
+    b = FastMultipole3d(*args, N=N, tree_depth=depth, ctx=rotation)
+    self_term = 0.0 if nt else q * 1e4
+    assert rel_l2(a.potentials - self_term, b.potentials - self_term) < TOL
+    assert rel_l2(a.forces, b.forces) < TOL
+
+
+@pytest.mark.parametrize("precision,bar", [("fp64", 5e-12), ("mixed", 1e-6)])
+@pytest.mark.parametrize("N", [2, 4, 7])
+def test_low_orders_in_a_forest(ctx, N, precision, bar):
+    """Nine problems of at most 512 finest cells: together their level 3 is above the
+    line (dense; FP32 expansions widened and rounded back), alone below it
+    (factored).  Bars of the scaled FP64 form and of the mixed form."""
+    problems = [uniform3d(4000, seed=60 + k) for k in range(9)]
+    kw = dict(N=N, tree_depth=4, max_leaf=2, ctx=ctx)
+    for (src, q), (pot, fld) in zip(problems, solve_batch(problems, precision=precision, **kw)):
+        b = FastMultipole3d((src, q), **kw)
+        assert rel_l2(pot - q * 1e4, b.potentials - q * 1e4) < bar
+        assert rel_l2(fld, b.forces) < bar
