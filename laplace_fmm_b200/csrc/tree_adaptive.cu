@@ -315,10 +315,11 @@ __global__ void uw_many_kernel(DevTree a, int pass, uint32_t* __restrict__ ucnt,
 	if (!pass) { ucnt[li] = nu; wcnt[li] = nw; }
 }
 
-// The line between them (B200, both passes): 3D 99 us a warp per leaf against
-// 207 a thread per leaf at 57,008 leaves, slower at 514,046; 2D (eight
-// colleagues) 537 against 82 on the 4.2M clustered set.
-template <int DIM> constexpr size_t uw_many() { return DIM == 3 ? 262144 : 16384; }
+// The line between them (B200, both passes, a warp per leaf against a thread per
+// leaf, us): 3D clustered 97 / 191 at 56,049 leaves, 150 / 247 at 84,635, 442 /
+// 308 at 240,441, 742 / 363 at 446,242; 3D uniform 48 / 37 at 32,768, 360 / 118
+// at 262,144; 2D (eight colleagues) 537 / 82 on the 4.2M clustered set.
+template <int DIM> constexpr size_t uw_many() { return DIM == 3 ? 131072 : 16384; }
 
 template <int DIM>
 void launch_uw(const DevTree& a, int pass, uint32_t* ucnt, uint32_t* wcnt, unsigned* flags, cudaStream_t s)
