@@ -113,13 +113,12 @@ __global__ void direct_reduce_kernel(size_t nt, int S, const double* __restrict_
 }
 
 // Target i against the sources of its own segment [poff[seg[i]], poff[seg[i] + 1])
-// (the sampled checks of a batch of problems in one launch): one block per
-// DSEG targets, the threads splitting the segment's sources, then a block
-// reduction in fixed order; neighbouring targets of one segment share the
-// reads of its sources (the checks of 256 problems: 10.6 ms with one target per
-// block, 8.3 with 4, 10.4 with 8).  3D, 1/r as in the FAST sums.
-constexpr int DSEG = 4;
-
+// (the sampled checks of a batch of problems in one launch): one block per D
+// targets, the threads splitting the segment's sources, then a block
+// reduction in fixed order (the same for every D); with D > 1 neighbouring
+// targets of one segment share the reads of its sources.  3D, 1/r as in the
+// FAST sums.
+template <int D>
 __global__ void __launch_bounds__(DT) direct_segments_kernel(const double* __restrict__ src,
                                                              const double* __restrict__ q,
                                                              const uint32_t* __restrict__ poff,
@@ -127,15 +126,15 @@ __global__ void __launch_bounds__(DT) direct_segments_kernel(const double* __res
                                                              const double* __restrict__ tgt,
                                                              double* __restrict__ pot, double* __restrict__ fld)
 {
-	__shared__ double red[DT / 32][DSEG][4];
-	const size_t i0 = (size_t)blockIdx.x * DSEG, i1 = min(m, i0 + DSEG);
+	__shared__ double red[DT / 32][D][4];
+	const size_t i0 = (size_t)blockIdx.x * D, i1 = min(m, i0 + D);
 	for (size_t a = i0; a < i1;) {             // runs of one segment
 		const int k = seg[a];
 		size_t b = a + 1;
 		while (b < i1 && seg[b] == k) ++b;
-		double x[DSEG][3], v[DSEG][4];
+		double x[D][3], v[D][4];
 #pragma unroll
-		for (int u = 0; u < DSEG; ++u) {
+		for (int u = 0; u < D; ++u) {
 			const size_t i = min(a + u, b - 1);
 #pragma unroll
 			for (int c = 0; c < 3; ++c) x[u][c] = tgt[3 * i + c];
@@ -145,7 +144,7 @@ __global__ void __launch_bounds__(DT) direct_segments_kernel(const double* __res
 		for (size_t j = poff[k] + threadIdx.x; j < hi; j += DT) {
 			const double sx = src[3 * j], sy = src[3 * j + 1], sz = src[3 * j + 2], sq = q[j];
 #pragma unroll
-			for (int u = 0; u < DSEG; ++u) {
+			for (int u = 0; u < D; ++u) {
 				if (a + u >= b) break;
 				const double dx = x[u][0] - sx, dy = x[u][1] - sy, dz = x[u][2] - sz;
 				const double inv = rsqrt_refined(fmax(dx * dx + dy * dy + dz * dz, FORCE_EPS2));
@@ -156,7 +155,7 @@ __global__ void __launch_bounds__(DT) direct_segments_kernel(const double* __res
 			}
 		}
 #pragma unroll
-		for (int u = 0; u < DSEG; ++u)
+		for (int u = 0; u < D; ++u)
 #pragma unroll
 			for (int c = 0; c < 4; ++c) {
 				double y = v[u][c];
@@ -165,7 +164,7 @@ __global__ void __launch_bounds__(DT) direct_segments_kernel(const double* __res
 			}
 		__syncthreads();
 		const int u = threadIdx.x >> 2, c = threadIdx.x & 3;
-		if (u < DSEG && a + u < b) {
+		if (u < D && a + u < b) {
 			double y = 0.0;
 			for (int w = 0; w < DT / 32; ++w) y += red[w][u][c];
 			if (c == 0) pot[a + u] = y;
@@ -182,7 +181,14 @@ int direct_segments_device(Context& ctx, const double* src, const double* q, con
                            const int32_t* seg, size_t m, const double* tgt, double* pot, double* fld)
 {
 	if (m == 0) return OK;
-	direct_segments_kernel<<<div_up(m, DSEG), DT, 0, ctx.stream>>>(src, q, poff, seg, m, tgt, pot, fld);
+	// Four targets per block once that leaves three blocks per SM (B200, one
+	// target per block against four: 10.6 ms / 8.3 for 32,768 samples of 256
+	// problems, 0.315 / 0.227 for 2,048 of 16; but 0.494 / 0.720 for 1,024 of
+	// 8, 9.6 / 14.2 for 512 of 4); eight take 10.4 for the 256 problems.
+	if (m >= (size_t)12 * ctx.num_sms)
+		direct_segments_kernel<4><<<div_up(m, 4), DT, 0, ctx.stream>>>(src, q, poff, seg, m, tgt, pot, fld);
+	else
+		direct_segments_kernel<1><<<(unsigned)m, DT, 0, ctx.stream>>>(src, q, poff, seg, m, tgt, pot, fld);
 	LFMM_CUDA(ctx, cudaGetLastError());
 	return OK;
 }
