@@ -113,6 +113,13 @@ int lfmm_check(lfmm_ctx* ctx);
  * check would (flags: bit mask, nonzero), so that callers can test their
  * handling of LFMM_ERR_DEVICE without a real failure. */
 int lfmm_debug_raise_flags(lfmm_ctx* ctx, unsigned flags);
+/* One leaf's multipole expansion (irregular 0, n_lists 1), or the local
+ * expansion of one cell from the sources of its X list's leaves (irregular 1),
+ * at the precision's expansions (FP64 or, mixed, FP32), for tests: sources
+ * [offsets[k], offsets[k + 1]) of list k, host arrays, positions in units of the
+ * cell's size about its centre; out: N (N + 1) / 2 pairs (re, im). */
+int lfmm_debug_leaf_sums(lfmm_ctx* ctx, int irregular, int N, int precision, size_t n_lists, const size_t* offsets,
+                         const double* xyz, const double* q, double* out);
 
 /* ---- 3D ----------------------------------------------------------------
  * Host buffers.  src_xyz: n_src x 3, src_q: n_src, tgt_xyz: n_tgt x 3 (or

@@ -19,7 +19,7 @@ STATUS = {0: "OK", -1: "ERR_ARG", -2: "ERR_CUDA", -3: "ERR_OOM", -4: "ERR_DEVICE
 # Every symbol include/lfmm.h declares (checked by the CPU tests).
 EXPORTS = [
     "lfmm_create", "lfmm_destroy", "lfmm_last_error", "lfmm_version", "lfmm_stream", "lfmm_check",
-    "lfmm_debug_raise_flags",
+    "lfmm_debug_raise_flags", "lfmm_debug_leaf_sums",
     "lfmm3d_solve", "lfmm3d_solve_device", "lfmm3d_solve_ex", "lfmm3d_solve_ex_device",
     "lfmm3d_solve_levels", "lfmm3d_solve_levels_device",
     "lfmm3d_solve_vector", "lfmm3d_solve_vector_device",
@@ -101,6 +101,7 @@ def load(path: Path | str = LIB_PATH):
         L.lfmm_stream.restype = P
         L.lfmm_check.argtypes = [P]
         L.lfmm_debug_raise_flags.argtypes = [P, ctypes.c_uint]
+        L.lfmm_debug_leaf_sums.argtypes = [P, I, I, I, SZ, P, P, P, P]
         solve = [P, SZ, P, P, SZ, P, I, I, D, I, P, P, ctypes.POINTER(LfmmStats)]
         for f in ("lfmm3d_solve", "lfmm3d_solve_device", "lfmm2d_solve", "lfmm2d_solve_device"):
             getattr(L, f).argtypes = solve

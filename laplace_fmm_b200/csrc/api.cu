@@ -462,6 +462,20 @@ int lfmm_debug_raise_flags(lfmm_ctx* ctx, unsigned flags)
 	return LFMM_OK;
 }
 
+int lfmm_debug_leaf_sums(lfmm_ctx* ctx, int irregular, int N, int precision, size_t n_lists, const size_t* offsets,
+                         const double* xyz, const double* q, double* out)
+{
+	if (!ctx || !offsets || !xyz || !q || !out || N < 1 || N > MAXN3 || n_lists < 1 || (!irregular && n_lists != 1) ||
+	    offsets[0] != 0)
+		return LFMM_ERR_ARG;
+	for (size_t k = 0; k < n_lists; ++k)
+		if (offsets[k + 1] < offsets[k] || offsets[k + 1] > 0x7fffffffull) return LFMM_ERR_ARG;
+	if (select_device(ctx)) return LFMM_ERR_CUDA;
+	return precision == LFMM_PRECISION_MIXED
+	           ? debug_leaf_sums<float>(ctx->c, irregular != 0, N, n_lists, offsets, xyz, q, out)
+	           : debug_leaf_sums<double>(ctx->c, irregular != 0, N, n_lists, offsets, xyz, q, out);
+}
+
 int lfmm_check(lfmm_ctx* ctx)
 {
 	if (!ctx) return LFMM_ERR_ARG;

@@ -58,15 +58,19 @@ __device__ __forceinline__ void reference_point(double& x, double& y, double z)
 // Eight lanes per particle, four particles per warp.  Lane l runs the chains
 // of the orders l, 15 - l and 16 + l one after another, so the coefficients
 // spread over the lanes (N = 16: 17 steps each) and every sum stays in a
-// register until the cell's last particle.  The first CHK steps of FP32 sums
-// (orders 0 to 7 up to CHK - 1 degrees above the order: the leaves' monopole
-// and dipole rounding errors would add up over the whole far field) are
-// compensated (Kahan).
+// register until the cell's last particle.  FP32 sums are compensated (Kahan):
+// the leaves' rounding errors would add up over the whole far field, and the
+// form before summed 32 particles in FP64 (orders 0 and 1) or in a tree.
+// Against it, single coefficients of leaves of 8 to 96 and of X lists of 60 to
+// 1,920 sources are off FP64 by 0.95 to 1.005 times as much (geometric means by
+// order and degree).  FP32 takes two particles per lane group at once for the
+// latencies of the compensation.
 // Issue bound.  A lane-per-particle form that summed the lanes' values through
 // shared memory took 840 M instructions and 1150 us for the P2L of 1,048,576
 // clustered particles at N = 16 (95.7k X entries), and 279 M for their P2M.
+// Compensating every step, not only the first six, takes the P2M of 16.8M
+// particles at N = 17 from 2.54 to 3.14 ms and their P2L from 5.2 to 6.2.
 constexpr int CHL = 8;
-constexpr int CHK = 6;
 // steps of the busiest lane (N = 17: 20, N = 18: 23)
 __host__ __device__ constexpr int chain_steps(int N) { return N <= 15 ? N : N == 16 ? 17 : N == 17 ? 20 : 23; }
 
@@ -93,47 +97,54 @@ __device__ __forceinline__ void chain_tab_fill(ChainTab<real>& tb, int N, int ti
 	for (int m = tid; m < N; m += nt) tb.S[m] = FarTab<real>::S(m);
 }
 
-// Sums of a cell: acc (FP32: minus comp) over the particles of a lane group.
+// Sums of a cell over the particles of a lane group: a (FP32: plus c, what the
+// additions to a have rounded off).
 template <typename real, int STEPS> struct ChainAcc {
 	typename V2<real>::t a[STEPS];
-	typename V2<real>::t c[CHK];       // FP32 compensation
+	typename V2<real>::t c[STEPS];     // FP32 compensation
 	__device__ __forceinline__ void clear()
 	{
 #pragma unroll
-		for (int s = 0; s < STEPS; ++s) a[s] = V2<real>::make(0, 0);
-		if constexpr (sizeof(real) == sizeof(float)) {
-#pragma unroll
-			for (int s = 0; s < CHK; ++s) c[s] = make_float2(0.f, 0.f);
+		for (int s = 0; s < STEPS; ++s) {
+			a[s] = V2<real>::make(0, 0);
+			if constexpr (sizeof(real) == sizeof(float)) c[s] = make_float2(0.f, 0.f);
 		}
 	}
 };
 
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+// a + c gains y - c (Kahan): y holds what is to be added and c
+__device__ __forceinline__ void kahan(float2& a, float2& c, float2 y)
+{
+	const float2 t = add2(a, y);
+	c = sub2(y, sub2(t, a));
+	a = t;
+}
 
 template <typename real>
 __device__ __forceinline__ typename V2<real>::t cm(typename V2<real>::t a, typename V2<real>::t b)
 { return V2<real>::make(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 
-// One particle per lane group added: q B_nm(x, y, z) (conjugated when stored).
-template <bool IRR, typename real, int STEPS>
-__device__ __forceinline__ void chain_add(ChainAcc<real, STEPS>& A, const ChainTab<real>& tb, real q, real x, real y,
-                                          real z, int N)
-{
+// One particle's chains on a lane: c = B_nm(x, y, z) at the lane's current step
+// (the sums are conjugated when stored).
+template <bool IRR, typename real, int STEPS> struct Chain {
 	using v2 = typename V2<real>::t;
-	const int l = threadIdx.x & (CHL - 1);
-	const real r2 = x * x + y * y + z * z;
-	const real ir2 = IRR ? real(1) / r2 : real(0);
-	const real b0 = IRR ? q * rsq<real>(r2) : q;
-	const v2 w = V2<real>::make(IRR ? x * ir2 : x, IRR ? y * ir2 : y);
-	const v2 w2 = cm<real>(w, w), w4 = cm<real>(w2, w2), one = V2<real>::make(1, 0);
-	// w^l and w^(7 - l)
-	v2 up = (l & 1) ? w : one, dn = (l & 1) ? one : w;
-	if (l & 2) up = cm<real>(up, w2); else dn = cm<real>(dn, w2);
-	if (l & 4) up = cm<real>(up, w4); else dn = cm<real>(dn, w4);
-	const int l1 = N - l, l12 = l1 + N - 15 + l;
-	v2 c, p = V2<real>::make(0, 0), c2 = p, c3 = p;
+	real z, r2;                        // IRR: 1 / r^2
+	v2 c, p, c2, c3;                   // this degree, the one below; the starts of chains 2 and 3
+	__device__ __forceinline__ void start(const ChainTab<real>& tb, real x, real y, real z_, int l, int N)
 	{
+		z = z_;
+		const real rr = x * x + y * y + z * z;
+		r2 = IRR ? real(1) / rr : rr;
+		const real b0 = IRR ? rsq<real>(rr) : real(1);
+		const v2 w = V2<real>::make(IRR ? x * r2 : x, IRR ? y * r2 : y);
+		const v2 w2 = cm<real>(w, w), w4 = cm<real>(w2, w2), one = V2<real>::make(1, 0);
+		// w^l and w^(7 - l)
+		v2 up = (l & 1) ? w : one, dn = (l & 1) ? one : w;
+		if (l & 2) up = cm<real>(up, w2); else dn = cm<real>(dn, w2);
+		if (l & 4) up = cm<real>(up, w4); else dn = cm<real>(dn, w4);
+		p = c2 = c3 = V2<real>::make(0, 0);
 		const real s1 = l < N ? b0 * tb.S[l] : real(0);
 		c = V2<real>::make(up.x * s1, up.y * s1);
 		if (STEPS > 8) {
@@ -150,41 +161,76 @@ __device__ __forceinline__ void chain_add(ChainAcc<real, STEPS>& A, const ChainT
 			}
 		}
 	}
-	const int T = chain_steps(N);
+	// the start of chain 2 or 3 at step s (l1, l12: the steps where they begin);
+	// chain 2 starts at step N - l >= N - 7, chain 3 at 2 N - 15 (N = 17, 18)
+	__device__ __forceinline__ void enter(int s, int l1, int l12)
+	{
+		if (STEPS > 8 && s >= (STEPS > 17 ? 10 : STEPS > 12 ? 6 : 2) && s == l1) c = c2;
+		if (STEPS > 17 && (s == 19 || s == 21) && s == l12) c = c3;
+	}
+	__device__ __forceinline__ void next(v2 ab)
+	{
+		const real az = ab.x * z, bb = IRR ? ab.y : ab.y * r2;
+		real nx = fma(az, c.x, -bb * p.x), ny = fma(az, c.y, -bb * p.y);
+		if (IRR) { nx *= r2; ny *= r2; }
+		p = c; c = V2<real>::make(nx, ny);
+	}
+};
+
+// K particles per lane group added, q c in the fused multiply-adds that also
+// take up the compensation; with K = 2 the table is read once for both.
+template <bool IRR, typename real, int STEPS, int K>
+__device__ __forceinline__ void chain_add(ChainAcc<real, STEPS>& A, const ChainTab<real>& tb, const real (&q)[K],
+                                          const real (&x)[K], const real (&y)[K], const real (&z)[K], int N)
+{
+	const int l = threadIdx.x & (CHL - 1), l1 = N - l, l12 = l1 + N - 15 + l, T = chain_steps(N);
+	Chain<IRR, real, STEPS> h[K];
+#pragma unroll
+	for (int j = 0; j < K; ++j) h[j].start(tb, x[j], y[j], z[j], l, N);
 #pragma unroll
 	for (int s = 0; s < STEPS; ++s) {
 		if (s >= T) break;
-		// chain 2 starts at step N - l >= N - 7, chain 3 at 2 N - 15 (N = 17, 18)
-		if (STEPS > 8 && s >= (STEPS > 17 ? 10 : STEPS > 12 ? 6 : 2) && s == l1) c = c2;
-		if (STEPS > 17 && (s == 19 || s == 21) && s == l12) c = c3;
-		const v2 ab = tb.ab[s * CHL + l];
+		const typename V2<real>::t ab = tb.ab[s * CHL + l];
+#pragma unroll
+		for (int j = 0; j < K; ++j) h[j].enter(s, l1, l12);
 		if constexpr (sizeof(real) == sizeof(float)) {
-			if (s < CHK) {
-				const float2 yk = sub2(c, A.c[s]), t = add2(A.a[s], yk);
-				A.c[s] = sub2(sub2(t, A.a[s]), yk);
-				A.a[s] = t;
-			} else {
-				A.a[s] = add2(A.a[s], c);
-			}
+#pragma unroll
+			for (int j = 0; j < K; ++j)
+				kahan(A.a[s], A.c[s], __ffma2_rn(make_float2(q[j], q[j]), h[j].c, A.c[s]));
 		} else {
-			A.a[s].x += c.x; A.a[s].y += c.y;
+#pragma unroll
+			for (int j = 0; j < K; ++j) { A.a[s].x = fma(q[j], h[j].c.x, A.a[s].x); A.a[s].y = fma(q[j], h[j].c.y, A.a[s].y); }
 		}
-		const real az = ab.x * z, bb = IRR ? ab.y : ab.y * r2;
-		real nx = fma(az, c.x, -bb * p.x), ny = fma(az, c.y, -bb * p.y);
-		if (IRR) { nx *= ir2; ny *= ir2; }
-		p = c; c = V2<real>::make(nx, ny);
+#pragma unroll
+		for (int j = 0; j < K; ++j) h[j].next(ab);
 	}
 }
 
-// The first cnt lanes' particles (the others: q = 0), four at a time.
+// K particles of every lane group from the lanes r + group, r + 4 + group.
+template <bool IRR, typename real, int STEPS, int K>
+__device__ __forceinline__ void chain_take(ChainAcc<real, STEPS>& A, const ChainTab<real>& tb, real q, real x, real y,
+                                           real z, int r, int N)
+{
+	real qk[K], xk[K], yk[K], zk[K];
+#pragma unroll
+	for (int j = 0; j < K; ++j) {
+		const int f = r + 4 * j + (threadIdx.x & 31) / CHL;
+		qk[j] = __shfl_sync(0xffffffffu, q, f); xk[j] = __shfl_sync(0xffffffffu, x, f);
+		yk[j] = __shfl_sync(0xffffffffu, y, f); zk[j] = __shfl_sync(0xffffffffu, z, f);
+	}
+	chain_add<IRR, real, STEPS, K>(A, tb, qk, xk, yk, zk, N);
+}
+
+// The first cnt lanes' particles (the others: q = 0), eight at a time in FP32
+// and a rest of up to four, or four at a time.
 template <bool IRR, typename real, int STEPS>
 __device__ __forceinline__ void chain_add32(ChainAcc<real, STEPS>& A, const ChainTab<real>& tb, real q, real x, real y,
                                             real z, int cnt, int N)
 {
-	const int gr = (threadIdx.x & 31) / CHL;
-	for (int r = 0; r < cnt; r += 32 / CHL)
-		chain_add<IRR, real, STEPS>(A, tb, __shfl_sync(0xffffffffu, q, r + gr), __shfl_sync(0xffffffffu, x, r + gr),
-		                            __shfl_sync(0xffffffffu, y, r + gr), __shfl_sync(0xffffffffu, z, r + gr), N);
+	int r = 0;
+	if constexpr (sizeof(real) == sizeof(float))
+		for (; r + 4 < cnt; r += 8) chain_take<IRR, real, STEPS, 2>(A, tb, q, x, y, z, r, N);
+	for (; r < cnt; r += 4) chain_take<IRR, real, STEPS, 1>(A, tb, q, x, y, z, r, N);
 }
 
 // The four lane groups' sums added up (every lane ends with its steps'
@@ -204,19 +250,15 @@ __device__ __forceinline__ void chain_reduce(ChainAcc<real, STEPS>& A, int N)
 			if constexpr (sizeof(real) == sizeof(float)) {
 				const float2 a = A.a[s], u = add2(a, b);
 				A.a[s] = u;
-				if (s < CHK) {
-					const float2 d = make_float2(__shfl_xor_sync(0xffffffffu, A.c[s].x, o),
-					                             __shfl_xor_sync(0xffffffffu, A.c[s].y, o));
-					const float2 bv = sub2(u, a), err = add2(sub2(a, sub2(u, bv)), sub2(b, bv));
-					A.c[s] = sub2(add2(A.c[s], d), err);
-				}
+				const float2 d = make_float2(__shfl_xor_sync(0xffffffffu, A.c[s].x, o),
+				                             __shfl_xor_sync(0xffffffffu, A.c[s].y, o));
+				const float2 bv = sub2(u, a), err = add2(sub2(a, sub2(u, bv)), sub2(b, bv));
+				A.c[s] = add2(add2(A.c[s], d), err);
 			} else {
 				A.a[s].x += b.x; A.a[s].y += b.y;
 			}
 		}
-		if constexpr (sizeof(real) == sizeof(float)) {
-			if (s < CHK) A.a[s] = sub2(A.a[s], A.c[s]);
-		}
+		if constexpr (sizeof(real) == sizeof(float)) A.a[s] = add2(A.a[s], A.c[s]);
 	}
 }
 

@@ -45,6 +45,11 @@ int fmm3d_scaled_on_tree(Context& ctx, const DevTree& t, int N, int precision, d
 int plain_p2m(Context& ctx, const DevTree& t, int N, double2* outer);
 int plain_leaves(Context& ctx, const DevTree& t, int N, const double2* inner, double* pot, double* field);
 
+// One leaf's P2M or one cell's P2L alone (lfmm_debug_leaf_sums).
+template <typename real>
+int debug_leaf_sums(Context& ctx, bool irregular, int N, size_t n_lists, const size_t* off, const double* xyz,
+                    const double* q, double* out);
+
 // Dense FP64 M2L operators [343][MT][MT] for cell size h (h = 1: the
 // level-independent scaled operators), cached in the context.
 double* m2l_ops_fp64(Context& ctx, int N, double h);

@@ -149,7 +149,39 @@ void by_steps(int N, F go)
 	if (N <= 8) go(std::integral_constant<int, 8>());
 	else if (N <= 12) go(std::integral_constant<int, 12>());
 	else if (N <= 16) go(std::integral_constant<int, 17>());
+	else if (N <= 17) go(std::integral_constant<int, 20>());
 	else go(std::integral_constant<int, 23>());
+}
+
+// P2M of every leaf.
+template <typename real>
+void launch_p2m(Context& ctx, const DevTree& t, int N, typename V2<real>::t* outer)
+{
+	by_steps(N, [&](auto st_) {
+		p2m_scaled_kernel<real, decltype(st_)::value>
+			<<<std::min(div_up(t.nleaves, FWPB), 8u * (unsigned)ctx.num_sms), FWPB * 32, 0, ctx.stream>>>(t, N, outer);
+	});
+}
+
+// P2L of every X list.
+template <typename real>
+int launch_p2l(Context& ctx, const DevTree& t, int N, typename V2<real>::t* inner)
+{
+	cudaStream_t s = ctx.stream;
+	// counter, list of longs, list of shorts (at most one cell per entry)
+	const size_t nlong = t.n_x / FAR_SHORT + 1;
+	uint32_t* next = static_cast<uint32_t*>(ctx.arena.take(sizeof(uint32_t) * (nlong + t.n_x + 3)));
+	if (!next) { ctx.last_error = "scaled solve: allocation failed"; return ERR_OOM; }
+	uint32_t *longs = next + 1, *shorts = longs + 1 + nlong;
+	LFMM_CUDA(ctx, cudaMemsetAsync(next, 0, 2 * sizeof(uint32_t), s));
+	LFMM_CUDA(ctx, cudaMemsetAsync(shorts, 0, sizeof(uint32_t), s));
+	x_select_kernel<<<div_up(t.ncells, 256), 256, 0, s>>>(t, shorts, longs);
+	by_steps(N, [&](auto st_) {
+		p2l_kernel<real, decltype(st_)::value><<<8 * ctx.num_sms, FWPB * 32, 0, s>>>(t, N, inner, next, shorts);
+		p2l_long_kernel<real, decltype(st_)::value><<<2 * ctx.num_sms, FWL * 32, 0, s>>>(t, N, inner, longs);
+	});
+	LFMM_CUDA(ctx, cudaGetLastError());
+	return OK;
 }
 
 // The dense FP64 M2L of a level (m2l_dense64); FP32 expansions are widened
@@ -196,11 +228,7 @@ int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, S
 	LFMM_CUDA(ctx, cudaMemsetAsync(outer, 0, sizeof(v2) * C * Nx2, s));
 	LFMM_CUDA(ctx, cudaMemsetAsync(inner, 0, sizeof(v2) * C * Nx2, s));
 	const unsigned resident = 8u * (unsigned)ctx.num_sms;
-	if (t.depth > 2)                       // multipoles below level 2 reach nothing
-		by_steps(N, [&](auto st_) {
-			p2m_scaled_kernel<real, decltype(st_)::value>
-				<<<std::min(div_up(t.nleaves, FWPB), resident), FWPB * 32, 0, s>>>(t, N, outer);
-		});
+	if (t.depth > 2) launch_p2m<real>(ctx, t, N, outer);   // multipoles below level 2 reach nothing
 	int st;
 	// the tensor-core engine on the FP32 expansions' larger levels (M2L; M2M
 	// through dense scaled operators, one per child octant)
@@ -260,20 +288,7 @@ int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, S
 			}
 		}
 	}
-	if (t.adaptive && t.n_x > 0) {
-		// counter, list of longs, list of shorts (at most one cell per entry)
-		const size_t nlong = t.n_x / FAR_SHORT + 1;
-		uint32_t* next = static_cast<uint32_t*>(ctx.arena.take(sizeof(uint32_t) * (nlong + t.n_x + 3)));
-		if (!next) { ctx.last_error = "scaled solve: allocation failed"; return ERR_OOM; }
-		uint32_t *longs = next + 1, *shorts = longs + 1 + nlong;
-		LFMM_CUDA(ctx, cudaMemsetAsync(next, 0, 2 * sizeof(uint32_t), s));
-		LFMM_CUDA(ctx, cudaMemsetAsync(shorts, 0, sizeof(uint32_t), s));
-		x_select_kernel<<<div_up(C, 256), 256, 0, s>>>(t, shorts, longs);
-		by_steps(N, [&](auto st_) {
-			p2l_kernel<real, decltype(st_)::value><<<resident, FWPB * 32, 0, s>>>(t, N, inner, next, shorts);
-			p2l_long_kernel<real, decltype(st_)::value><<<2 * ctx.num_sms, FWL * 32, 0, s>>>(t, N, inner, longs);
-		});
-	}
+	if (t.adaptive && t.n_x > 0 && (st = launch_p2l<real>(ctx, t, N, inner))) return st;
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[3], s));
 	for (int L = 3; L < t.depth; ++L) {
 		if (t.lsize[L] == 0) continue;
@@ -309,6 +324,57 @@ int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, S
 
 } // namespace
 
+// P2M of one leaf, or P2L of one cell, from the sources of n_lists lists (P2M:
+// one list), given in the scaled frame of the leaf or cell; out: the N (N + 1) / 2
+// coefficients (re, im), widened to FP64.
+template <typename real>
+int debug_leaf_sums(Context& ctx, bool irregular, int N, size_t n_lists, const size_t* off, const double* xyz,
+                    const double* q, double* out)
+{
+	using v2 = typename V2<real>::t;
+	if (int st = upload_scaled_constants(ctx)) return st;
+	cudaStream_t s = ctx.stream;
+	const size_t n = off[n_lists], C = n_lists + 1, Nx2 = (size_t)N * (N + 1) / 2;
+	// cell 0: the leaf or cell, of size 1 about the origin; cells 1 ..: the lists
+	std::vector<double> xs(4 * n);
+	for (size_t i = 0; i < n; ++i) { for (int d = 0; d < 3; ++d) xs[d * n + i] = xyz[3 * i + d]; xs[3 * n + i] = q[i]; }
+	std::vector<uint32_t> u(2 * C + C + 1);
+	std::vector<int32_t> idx(C);
+	u[0] = 0; u[C] = (uint32_t)n;
+	for (size_t k = 1; k < C; ++k) { u[k] = (uint32_t)off[k - 1]; u[C + k] = (uint32_t)off[k]; idx[k - 1] = (int32_t)k; }
+	for (size_t k = 0; k <= C; ++k) u[2 * C + k] = k ? (uint32_t)n_lists : 0u;
+	ctx.arena.reset();
+	double* x = static_cast<double*>(ctx.arena.take(sizeof(double) * (4 * n + 3)));
+	uint32_t* du = static_cast<uint32_t*>(ctx.arena.take(sizeof(uint32_t) * u.size()));
+	int32_t* di = static_cast<int32_t*>(ctx.arena.take(sizeof(int32_t) * (C + 1)));
+	uint8_t* lev = static_cast<uint8_t*>(ctx.arena.take(C));
+	v2* e = static_cast<v2*>(ctx.arena.take(sizeof(v2) * Nx2));
+	if (!x || !du || !di || !lev || !e) { ctx.last_error = "leaf sums: allocation failed"; return ERR_OOM; }
+	LFMM_CUDA(ctx, cudaMemcpyAsync(x, xs.data(), sizeof(double) * xs.size(), cudaMemcpyHostToDevice, s));
+	LFMM_CUDA(ctx, cudaMemsetAsync(x + 4 * n, 0, 3 * sizeof(double), s));
+	LFMM_CUDA(ctx, cudaMemcpyAsync(du, u.data(), sizeof(uint32_t) * u.size(), cudaMemcpyHostToDevice, s));
+	LFMM_CUDA(ctx, cudaMemcpyAsync(di, idx.data(), sizeof(int32_t) * C, cudaMemcpyHostToDevice, s));
+	LFMM_CUDA(ctx, cudaMemsetAsync(di + C, 0, sizeof(int32_t), s));
+	LFMM_CUDA(ctx, cudaMemsetAsync(lev, 0, C, s));
+	LFMM_CUDA(ctx, cudaMemsetAsync(e, 0, sizeof(v2) * Nx2, s));
+	DevTree t;
+	t.n = n; t.ncells = 1; t.nleaves = 1; t.adaptive = true; t.n_x = n_lists; t.geo_host[3] = 1.0;
+	t.x = x; t.y = x + n; t.z = x + 2 * n; t.q = x + 3 * n;
+	t.cx = x + 4 * n; t.cy = x + 4 * n + 1; t.cz = x + 4 * n + 2;
+	t.pbeg = du; t.send = du + C; t.x_off = du + 2 * C; t.x_idx = di; t.leaves = di + C; t.lev = lev;
+	if (irregular) {
+		if (int st = launch_p2l<real>(ctx, t, N, e)) return st;
+	} else {
+		launch_p2m<real>(ctx, t, N, e);
+	}
+	std::vector<v2> h(Nx2);
+	LFMM_CUDA(ctx, cudaMemcpyAsync(h.data(), e, sizeof(v2) * Nx2, cudaMemcpyDeviceToHost, s));
+	LFMM_CUDA(ctx, cudaStreamSynchronize(s));
+	for (size_t c = 0; c < Nx2; ++c) { out[2 * c] = h[c].x; out[2 * c + 1] = h[c].y; }
+	ctx.arena.settle();
+	return OK;
+}
+
 int plain_p2m(Context& ctx, const DevTree& t, int N, double2* outer)
 {
 	if (int st = upload_scaled_constants(ctx)) return st;
@@ -333,6 +399,9 @@ int plain_leaves(Context& ctx, const DevTree& t, int N, const double2* inner, do
 	LFMM_CUDA(ctx, cudaGetLastError());
 	return OK;
 }
+
+template int debug_leaf_sums<float>(Context&, bool, int, size_t, const size_t*, const double*, const double*, double*);
+template int debug_leaf_sums<double>(Context&, bool, int, size_t, const size_t*, const double*, const double*, double*);
 
 float* m2l_ops_fp32(Context& ctx, int N)
 {
