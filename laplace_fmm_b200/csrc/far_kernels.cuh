@@ -44,7 +44,11 @@ template <> struct FarTab<double> {
 // FP64: the reference's spherical coordinates take r + 1e-12 as the radius and
 // cos t = z / (r + 1e-12) (common/simple_math.h:101-117), which moves a point
 // away from the z axis by rho'^2 = rho^2 + (2 r + 1e-12) 1e-12; the parity of
-// its outputs at 1e-12 needs the same point here.
+// the plain form's outputs at 1e-12 needs the same point here.  The scaled form
+// moves its targets too (the vector form is held to the reference at 1e-12), by
+// 1e-12 of the cell's size: a target exactly on the axis of its leaf or of a W
+// cell is evaluated up to 1e-6 cells beside it (at N = 18 up to 8e-7 of the field
+// at such a target of a clustered set, 6e-13 at the others).
 __device__ __forceinline__ void reference_point(double& x, double& y, double z)
 {
 	constexpr double e = 1e-12;
