@@ -73,9 +73,10 @@ __device__ __forceinline__ bool beyond_1e300(double x) { return (unsigned)__doub
 // 1 / sqrt(x), x > 0: the hardware's FP64 reciprocal square root approximation
 // (rsqrt.approx.ftz.f64, no FP32 round trip; measured seed error 2^-20.1)
 // refined by one third-order step of the binomial series (1 - r)^(-1/2) =
-// 1 + r/2 + 3r^2/8 + ..., r = 1 - x y^2 (measured 1.4e-16): a seed error e leaves
-// ~(5/16)(2e)^3, below FP64 rounding for e < 2^-18.  The FP64 square root and
-// divide above 1e300.
+// 1 + r/2 + 3r^2/8 + ..., r = 1 - x y^2: a seed error e leaves ~(5/16)(2e)^3, below
+// FP64 rounding for e < 2^-18, beside the roundings of x y (half of 2^-53) and of
+// the last sum (2^-53; measured 1.4e-16 in all).  The FP64 square root and divide
+// above 1e300.
 __device__ __forceinline__ double rsqrt_refined(double x)
 {
 	if (beyond_1e300(x)) return 1.0 / sqrt(x);
@@ -85,16 +86,19 @@ __device__ __forceinline__ double rsqrt_refined(double x)
 	return fma(y * r, fma(r, 0.375, 0.5), y);
 }
 
-// 1 / x, x > 0: the hardware's FP64 reciprocal approximation refined by the
-// geometric series 1 / (1 - e) = 1 + e + e^2 + ..., e = 1 - x y (a seed error
-// below 2^-18 leaves e^3 < 2^-54).  The FP64 divide above 1e300.
-__device__ __forceinline__ double recip_refined(double x)
+// q / x, x > 0; plain: |q| is below 1e300.  The hardware's FP64 reciprocal
+// approximation y (1 - x y = e) refined once, y (1 + e), off by e^2 < 2^-36 for a
+// seed error below 2^-18; then the quotient q y corrected by its remainder, which
+// leaves the rounding of the last sum (2^-72 before it).  The FP64 divide where q
+// or x is not below 1e300.
+__device__ __forceinline__ double quotient_refined(double q, double x, bool plain)
 {
-	if (beyond_1e300(x)) return 1.0 / x;
+	if (beyond_1e300(x) || !plain) return q / x;
 	double y;
 	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-	const double e = fma(-x, y, 1.0);
-	return fma(y, fma(e, e, e), y);
+	y = fma(y, fma(-x, y, 1.0), y);
+	const double p = q * y;
+	return fma(fma(-p, x, q), y, p);
 }
 
 // Spherical coordinates with the reference's conventions

@@ -307,10 +307,12 @@ __global__ void __launch_bounds__(WPB2 * 32) l2l2d_add_kernel(DevTree t, Exp2 E,
 // Leaves: P2P over the close list (the leaf itself first) and L2P
 // (reference cpu/multipole.cpp:233-449).  One warp per work unit, a leaf's
 // targets in chunks of 32 (so a crowded leaf of a clustered set spreads over
-// many warps; bound by the FP64 pipe, about 24 operations per pair: 1/r^2 by
-// recip_refined instead of a division took the leaves of 4.2M clustered
-// particles from 3.75 to 3.59 ms, eight conflict-free copies of a 129-entry
-// table with one more term of the series back to 3.75); a leaf of nt <= 16 targets is one unit whose warp runs TP = nt
+// many warps; bound by the FP64 pipe, about 24 operations per pair: q / r^2 by
+// quotient_refined instead of the division took the leaves of 4.2M clustered
+// particles from 3.75 to 3.66 ms; a reciprocal and a product, 3.54, round twice;
+// eight conflict-free copies of a 129-entry log table with one more term of the
+// series took 0.2 ms more, the distance clamp as an integer comparison 0.17); a
+// leaf of nt <= 16 targets is one unit whose warp runs TP = nt
 // rounded up to a power of two targets at once and splits the sources into
 // 32 / TP phases, summed by shuffles at the end.
 constexpr int LW2 = 4;
@@ -398,14 +400,16 @@ __global__ void __launch_bounds__(LW2 * 32) leaves2d_kernel(DevTree t, Exp2 E, c
 				if (pos >= ex && pos < inc) j = bg + (pos - ex);
 			}
 			__syncwarp();
-			if (lane < cnt) { sx[w][lane] = t.x[j]; sy[w][lane] = t.y[j]; sq[w][lane] = t.q[j]; }
+			const double qj = lane < cnt ? t.q[j] : 0.0;
+			if (lane < cnt) { sx[w][lane] = t.x[j]; sy[w][lane] = t.y[j]; sq[w][lane] = qj; }
+			const bool plain = !__any_sync(0xffffffffu, beyond_1e300(fabs(qj)));
 			__syncwarp();
 			if (valid) {
 				for (int k = ph; k < cnt; k += G) {
 					const double dx = xi - sx[w][k], dy = yi - sy[w][k];
 					const double r2 = fmax(dx * dx + dy * dy, FORCE_EPS2);
 					pot = fma(sq[w][k], log_table(r2, slog, ln2_hi, ln2_lo), pot);     // halved below
-					const double qr = sq[w][k] * recip_refined(r2);
+					const double qr = quotient_refined(sq[w][k], r2, plain);
 					fr = fma(dx, qr, fr); fi = fma(-dy, qr, fi);
 				}
 			}
@@ -583,14 +587,16 @@ __global__ void __launch_bounds__(LW2 * 32) leaves2d_adaptive_kernel(DevTree t, 
 			const uint32_t bg = __shfl_sync(FULL, cbeg, clo);
 			const uint32_t j = bg + (pos - (clo > 0 ? ex : 0u));
 			__syncwarp();
-			if (lane < cnt) { sx[w][lane] = t.x[j]; sy[w][lane] = t.y[j]; sq[w][lane] = t.q[j]; }
+			const double qj = lane < cnt ? t.q[j] : 0.0;
+			if (lane < cnt) { sx[w][lane] = t.x[j]; sy[w][lane] = t.y[j]; sq[w][lane] = qj; }
+			const bool plain = !__any_sync(0xffffffffu, beyond_1e300(fabs(qj)));
 			__syncwarp();
 			if (valid) {
 				for (int k = ph; k < cnt; k += G) {
 					const double dx = xi - sx[w][k], dy = yi - sy[w][k];
 					const double r2 = fmax(dx * dx + dy * dy, FORCE_EPS2);
 					pot = fma(sq[w][k], log_table(r2, slog, ln2_hi, ln2_lo), pot);     // halved below
-					const double qr = sq[w][k] * recip_refined(r2);
+					const double qr = quotient_refined(sq[w][k], r2, plain);
 					fr = fma(dx, qr, fr); fi = fma(-dy, qr, fi);
 				}
 			}
