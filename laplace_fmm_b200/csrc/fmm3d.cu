@@ -289,23 +289,25 @@ int upload_constants(Context& ctx)
 
 } // namespace
 
-// Dense FP64 M2L operators for cell size h, cached in the context.
+int m2l_ops_build(Context& ctx, int N, double h, double* out)
+{
+	const int MT = m2l_padded(N), R = N * (N + 1);
+	LFMM_CUDA(ctx, cudaMemsetAsync(out, 0, m2l_ops_bytes(N), ctx.stream));
+	m2l_ops_kernel<<<div_up((size_t)343 * R, WPB), WPB * 32, 0, ctx.stream>>>(N, MT, h, ctx.tables.d, out,
+	                                                                          ctx.dev_flags);
+	LFMM_CUDA(ctx, cudaGetLastError());
+	return OK;
+}
+
 double* m2l_ops_fp64(Context& ctx, int N, double h)
 {
 	for (auto& e : ctx.opcache)
 		if (e.N == N && e.prec == 0 && e.h == h) { e.stamp = ++ctx.opcache_clock; return static_cast<double*>(e.ptr); }
-	if (upload_constants(ctx)) return nullptr;
-	const int MT = m2l_padded(N), R = N * (N + 1);
-	size_t bytes = sizeof(double) * 343 * (size_t)MT * MT;
 	opcache_make_room(ctx);
 	OpCacheEntry e;
-	e.N = N; e.prec = 0; e.h = h; e.bytes = bytes; e.stamp = ++ctx.opcache_clock;
-	if (cudaMalloc(&e.ptr, bytes) != cudaSuccess) { cudaGetLastError(); ctx.last_error = "m2l operators: out of memory"; return nullptr; }
-	cudaMemsetAsync(e.ptr, 0, bytes, ctx.stream);
-	size_t tasks = (size_t)343 * R;
-	m2l_ops_kernel<<<div_up(tasks, WPB), WPB * 32, 0, ctx.stream>>>(N, MT, h, ctx.tables.d, static_cast<double*>(e.ptr),
-	                                                                 ctx.dev_flags);
-	if (cudaGetLastError() != cudaSuccess) { cudaFree(e.ptr); ctx.last_error = "m2l operators: launch failed"; return nullptr; }
+	e.N = N; e.prec = 0; e.h = h; e.bytes = m2l_ops_bytes(N); e.stamp = ++ctx.opcache_clock;
+	if (cudaMalloc(&e.ptr, e.bytes) != cudaSuccess) { cudaGetLastError(); ctx.last_error = "m2l operators: out of memory"; return nullptr; }
+	if (m2l_ops_build(ctx, N, h, static_cast<double*>(e.ptr))) { cudaFree(e.ptr); return nullptr; }
 	ctx.opcache.push_back(e);
 	return static_cast<double*>(e.ptr);
 }

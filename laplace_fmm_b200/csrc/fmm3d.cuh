@@ -1,6 +1,6 @@
 // 3D rotation-based Laplace FMM on the device (plain FP64 form).
 #pragma once
-#include "tree.cuh"
+#include "m2l_gemm.cuh"
 
 namespace lfmm {
 
@@ -51,7 +51,11 @@ int debug_leaf_sums(Context& ctx, bool irregular, int N, size_t n_lists, const s
                     const double* q, double* out);
 
 // Dense FP64 M2L operators [343][MT][MT] for cell size h (h = 1: the
-// level-independent scaled operators), cached in the context.
+// level-independent scaled operators): built into out (m2l_ops_bytes), which the
+// FP32 and tensor-core sets are converted from, or cached in the context (the
+// FP64 form's low orders, m2l_dense64).
+inline size_t m2l_ops_bytes(int N) { return sizeof(double) * 343 * (size_t)m2l_padded(N) * m2l_padded(N); }
+int m2l_ops_build(Context& ctx, int N, double h, double* out);
 double* m2l_ops_fp64(Context& ctx, int N, double h);
 float* m2l_ops_fp32(Context& ctx, int N);
 

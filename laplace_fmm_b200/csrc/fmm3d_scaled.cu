@@ -407,14 +407,28 @@ float* m2l_ops_fp32(Context& ctx, int N)
 {
 	for (auto& e : ctx.opcache)
 		if (e.N == N && e.prec == 1) { e.stamp = ++ctx.opcache_clock; return static_cast<float*>(e.ptr); }
-	double* d = m2l_ops_fp64(ctx, N, 1.0);
-	if (!d) return nullptr;
-	const int MT = m2l_padded(N);
-	size_t cnt = (size_t)343 * MT * MT;
+	const size_t bytes = m2l_ops_bytes(N), cnt = bytes / sizeof(double);
+	opcache_make_room(ctx);
 	OpCacheEntry e;
 	e.N = N; e.prec = 1; e.h = 1.0; e.bytes = cnt * sizeof(float); e.stamp = ++ctx.opcache_clock;
-	if (cudaMalloc(&e.ptr, e.bytes) != cudaSuccess) { cudaGetLastError(); ctx.last_error = "m2l operators: out of memory"; return nullptr; }
-	convert_kernel<<<div_up(cnt, 256), 256, 0, ctx.stream>>>(d, static_cast<float*>(e.ptr), cnt);
+	double* d = nullptr;
+	if (cudaMalloc(&d, bytes) != cudaSuccess || cudaMalloc(&e.ptr, e.bytes) != cudaSuccess) {
+		cudaGetLastError();
+		cudaFree(d);
+		ctx.last_error = "m2l operators: out of memory";
+		return nullptr;
+	}
+	bool ok = m2l_ops_build(ctx, N, 1.0, d) == OK;
+	if (ok) {
+		convert_kernel<<<div_up(cnt, 256), 256, 0, ctx.stream>>>(d, static_cast<float*>(e.ptr), cnt);
+		ok = cudaStreamSynchronize(ctx.stream) == cudaSuccess;
+	}
+	cudaFree(d);
+	if (!ok) {
+		cudaFree(e.ptr);
+		ctx.last_error = "m2l operators: build failed";
+		return nullptr;
+	}
 	ctx.opcache.push_back(e);
 	return static_cast<float*>(e.ptr);
 }

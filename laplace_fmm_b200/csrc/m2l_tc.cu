@@ -1151,50 +1151,48 @@ const uint4* m2l_ops_tc(Context& ctx, int N, float* t_inv)
 			if (t_inv) *t_inv = e.aux;
 			return static_cast<const uint4*>(e.ptr);
 		}
-	const double* d = m2l_ops_fp64(ctx, N, 1.0);
-	if (!d) return nullptr;
 	const int NC = m2l_padded(N), R = N * (N + 1), NA = m2l_tc_drained(N);
 	const int KB = f16 ? (NC + 63) / 64 : m2l_tc_kblocks(N);
+	opcache_make_room(ctx);
 	OpCacheEntry e;
 	e.N = N; e.prec = prec; e.h = 1.0; e.stamp = ++ctx.opcache_clock;
-	double scale = 1.0;
-	if (f16) {
-		// the largest operator magnitude scaled into [2^14, 2^15)
-		unsigned long long* mx = static_cast<unsigned long long*>(ctx.arena.take(sizeof(unsigned long long)));
-		if (!mx) { ctx.last_error = "tensor-core operators: allocation failed"; return nullptr; }
-		const size_t n = (size_t)343 * NC * NC;
-		unsigned long long hb = 0;
-		if (cudaMemsetAsync(mx, 0, sizeof(hb), ctx.stream) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-		absmax64_kernel<<<(unsigned)std::min<size_t>(div_up(n, 256), 8 * (size_t)ctx.num_sms), 256, 0, ctx.stream>>>(
-			d, n, mx);
-		if (cudaMemcpyAsync(&hb, mx, sizeof(hb), cudaMemcpyDeviceToHost, ctx.stream) != cudaSuccess ||
-		    cudaStreamSynchronize(ctx.stream) != cudaSuccess) {
-			cudaGetLastError();
-			ctx.last_error = "tensor-core operators: scale reduction failed";
-			return nullptr;
-		}
-		double m;
-		std::memcpy(&m, &hb, sizeof(m));
-		const int ex = m > 0.0 ? std::ilogb(m) : 0;
-		scale = std::ldexp(1.0, 14 - ex);
-		e.aux = (float)std::ldexp(1.0, ex - 14);
-	}
 	e.bytes = f16 ? tc16_ops_bytes(343, N) : tc_ops_bytes(343, N);
-	if (cudaMalloc(&e.ptr, e.bytes) != cudaSuccess) {
+	double* d = nullptr;                       // the FP64 operators, and a word for their largest magnitude
+	if (cudaMalloc(&d, m2l_ops_bytes(N) + sizeof(unsigned long long)) != cudaSuccess ||
+	    cudaMalloc(&e.ptr, e.bytes) != cudaSuccess) {
 		cudaGetLastError();
+		cudaFree(d);
 		ctx.last_error = "tensor-core operators: out of memory";
 		return nullptr;
 	}
-	const size_t threads = (size_t)343 * KB * NC * 32;
-	if (f16)
-		build_tc16_ops_kernel<<<div_up(threads, 256), 256, 0, ctx.stream>>>(d, 343, NC, NA, R, KB, scale,
-		                                                                    static_cast<uint32_t*>(e.ptr));
-	else
-		build_tc_ops_kernel<<<div_up(threads, 256), 256, 0, ctx.stream>>>(d, 343, NC, NA, R, KB,
-		                                                                  static_cast<uint32_t*>(e.ptr));
-	if (cudaGetLastError() != cudaSuccess) {
+	auto build = [&]() -> int {
+		const size_t n = (size_t)343 * NC * NC, threads = (size_t)343 * KB * NC * 32;
+		if (int st = m2l_ops_build(ctx, N, 1.0, d)) return st;
+		if (f16) {
+			// the largest operator magnitude scaled into [2^14, 2^15)
+			unsigned long long* mx = reinterpret_cast<unsigned long long*>(d + n);
+			double m = 0.0;
+			LFMM_CUDA(ctx, cudaMemsetAsync(mx, 0, sizeof(m), ctx.stream));
+			absmax64_kernel<<<(unsigned)std::min<size_t>(div_up(n, 256), 8 * (size_t)ctx.num_sms), 256, 0, ctx.stream>>>(
+				d, n, mx);
+			LFMM_CUDA(ctx, cudaMemcpyAsync(&m, mx, sizeof(m), cudaMemcpyDeviceToHost, ctx.stream));
+			LFMM_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
+			const int ex = m > 0.0 ? std::ilogb(m) : 0;
+			e.aux = (float)std::ldexp(1.0, ex - 14);
+			build_tc16_ops_kernel<<<div_up(threads, 256), 256, 0, ctx.stream>>>(d, 343, NC, NA, R, KB, std::ldexp(1.0, 14 - ex),
+			                                                                    static_cast<uint32_t*>(e.ptr));
+		} else {
+			build_tc_ops_kernel<<<div_up(threads, 256), 256, 0, ctx.stream>>>(d, 343, NC, NA, R, KB,
+			                                                                  static_cast<uint32_t*>(e.ptr));
+		}
+		LFMM_CUDA(ctx, cudaGetLastError());
+		LFMM_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
+		return OK;
+	};
+	const int st = build();
+	cudaFree(d);
+	if (st) {
 		cudaFree(e.ptr);
-		ctx.last_error = "tensor-core operators: launch failed";
 		return nullptr;
 	}
 	ctx.opcache.push_back(e);

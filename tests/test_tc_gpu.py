@@ -141,3 +141,22 @@ def test_autotuned_split_matches_fixed_rule(ctx):
     assert rel_l2(noself(a.potentials, q), noself(b.potentials, q)) < 5e-7
     assert rel_l2(a.forces, b.forces) < 5e-7
     fixed.close()
+
+
+@pytest.mark.parametrize("name,var,kept", [("f16", "LFMM_M2L_TYPE", 343 * (6 * 352 + 3 * 160) * 128),
+                                           ("tf32", "LFMM_M2L_TYPE", 343 * (11 * 352 + 5 * 160) * 128),
+                                           ("simt", "LFMM_M2L", 343 * 272 * 272 * 4)])
+def test_operators_kept(name, var, kept):
+    """A context keeps the converted operators of an order (N = 18; the SIMT
+    engine's of N = 16) and gives the FP64 ones back that they were made from
+    (340 MB at N = 18, 203 MB at N = 16)."""
+    import torch
+    c = engine_context(name, var)
+    src, q = uniform3d(30000, seed=3)
+    kw = dict(tree_depth=5, precision="mixed", ctx=c)
+    FastMultipole3d((src, q), N=7, **kw)
+    free = torch.cuda.mem_get_info(0)[0]
+    FastMultipole3d((src, q), N=16 if name == "simt" else 18, **kw)
+    used = free - torch.cuda.mem_get_info(0)[0]
+    c.close()
+    assert kept <= used < kept + 120e6
