@@ -282,52 +282,15 @@ def tf32_peak_tflops(torch):
     return 2 * 8192 ** 3 / (best * 1e-3) / 1e12
 
 
-def launches_per_solve(depth, dim, radix_passes, adaptive, precision, learned=False, parts=False):
-    """Kernels the library enqueues for one solve (tree + FMM passes), counted
-    from the launch sites; the learned solve adds its features (far strength
-    per level, accumulation per level, leaf features), the network, the
-    prediction sums, the sampled direct sum (split kernel and reduction) and
-    the RMS and error sums.  A trace of the 16.8M-particle learned solve shows
-    294 kernels per solve; this count of 283 leaves out the leaf-size
-    candidates' counts and the autotuned split reductions."""
-    extra = (1 + (depth - 2) + (depth - 1) + 1 + 1 + 1 + 2 + 1 + 1) if learned else 0
-    scan = 3
-    tree = 2 + 1 + radix_passes * (1 + scan + 1) + 1 + 1 + scan + 1 + 1
-    tree += (depth - 1) * (1 + scan + 1 + 1) + depth + 1
-    lists = depth - 1
-    if adaptive or precision != "fp64":
-        tree += depth + depth * (1 + scan) + depth + 1 + scan + 1 + 1 + lists + 2 + 2 + 3 * scan
-        # plan (class count, scatter, slot table) + translation per level,
-        # split reductions on levels 2-3, the mixed form's source staging
-        # (largest magnitude, split) on the finer ones
-        m2l = max(0, depth - 2) * (3 + 1) + 2 + (2 * max(0, depth - 4) if precision == "mixed" else 0)
-        m2m = 2 * max(0, depth - 3)                # plan + translation, levels depth-2 .. 2
-        # P2M, axial tables; P2L: list selection, short and long lists; L2L;
-        # near field, expansions of the leaves with short and with long lists
-        fmm = 1 + 1 + m2m + m2l + 3 + max(0, depth - 3) + 3
-        return (tree, fmm) if parts else tree + fmm + extra
-    if adaptive and dim == 2:
-        tree += depth + depth * (1 + scan) + depth + 1 + scan + 1 + 1 + lists + 2 + 2 + 3 * scan
-        # P2M, M2M per level, per M2L level: class count, scatter, slot table,
-        # Hankel M2L (+ a split reduction on the small levels); P2L, L2L adds,
-        # leaf work units (count + scan) and the leaves
-        levels = max(0, depth - 2)
-        split = sum(1 for L in range(2, depth) if 4 ** L < 37000)
-        fmm = 1 + (depth - 1) + 4 * levels + split + 1 + max(0, depth - 3) + 1 + scan + 1
-        return (tree, fmm) if parts else tree + fmm
-    tree += lists
-    if dim == 3:
-        # P2M, axial tables, M2M (plan + translation), M2L, L2L, leaves
-        fmm = 1 + 1 + 2 * max(0, depth - 3) + max(0, depth - 2) * 5 + max(0, depth - 3) + 1
-    else:
-        # per level 2..depth-1: class count, scatter, slot table, Hankel M2L,
-        # and a split reduction on the levels too small to fill the GPU
-        # (fewer than ~37k cells: levels up to 7); L2L adds; leaf work units
-        # (count + scan) and the leaves
-        levels = max(0, depth - 2)
-        split = sum(1 for L in range(2, depth) if 4 ** L < 37000)
-        fmm = 1 + (depth - 1) + 4 * levels + split + max(0, depth - 3) + 1 + scan + 1
-    return tree + fmm
+def traced_launches(torch, solve):
+    """The library's kernels that one call of solve launches, from a trace of
+    one call (taken after the timed region)."""
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        solve()
+        torch.cuda.synchronize()
+    return sum(1 for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA and "lfmm::" in e.name)
 
 
 # ---------------------------------------------------------------- ours
@@ -552,7 +515,8 @@ def run_ours(args, cfg, rank, world, local_rank):
                "h2d_bytes_per_step": int(h_src.numel() * 8 + h_q.numel() * 8),
                "d2h_bytes_per_step": int(h_pot.numel() * 8 + h_fld.numel() * 8)}
     return dict(ms=ms, stats=stats, acc=acc, e2e=e2e, clocks=clk.summary(), torch=torch, dist=dist, ctx=ctx,
-                plain=plain, learned=dict(info_box) if learned else None, plan=plan_line, mixed_fixed=mixed_fixed)
+                plain=plain, learned=dict(info_box) if learned else None, plan=plan_line, mixed_fixed=mixed_fixed,
+                launches=traced_launches(torch, step_dev))
 
 
 def m2l_flops(N):
@@ -625,17 +589,16 @@ def roofline(cfg, stats, peaks, fp64_tflops, fp32_tflops, tf32_tflops, phase=Non
     fp64 = cfg["precision"] == "fp64"
     if dom == "m2l" and cfg["dim"] == 2:
         # 2D: one complex N x N operator per far pair, 8 N^2 real flops; the
-        # GEMMs run it as a real MT x MT block (MT = 2N rounded up to 16)
+        # Hankel form multiplies two real columns by N x N (padded to 8 x 4 tiles)
         ms_k = stats.get("ms_m2l_kernel") or ms
         N = cfg["N"]
-        mt = (2 * N + 15) // 16 * 16
         flops = 8.0 * N * N * stats["n_far_pairs"]
-        executed = 2.0 * mt * mt * stats["n_far_pairs"]
+        executed = 4.0 * ((N + 7) // 8 * 8) * ((N + 3) // 4 * 4) * stats["n_far_pairs"]
         achieved = flops / (ms_k * 1e-3) / 1e12
-        return {"kernel": "m2l_gemm_kernel<double, *, 4, 2> (2D FP64 GEMMs by quadrant class and offset)",
+        return {"kernel": "m2l2d_hankel_kernel (2D FP64, by quadrant class and offset)",
                 "bound": "fp64", "achieved": achieved, "peak": fp64_tflops, "unit": "TFLOP/s",
                 "frac": achieved / fp64_tflops, "peak_source": "measured cuBLAS DGEMM", "algorithmic_flops": flops,
-                "executed_dense_flops": executed, "executed_tflops": executed / (ms_k * 1e-3) / 1e12,
+                "executed_flops": executed, "executed_tflops": executed / (ms_k * 1e-3) / 1e12,
                 "kernel_ms": ms_k, "kernel_launches": stats.get("n_m2l_kernel", 0), "phase_ms": phases["m2l"],
                 "traffic": None}
     if dom == "m2l" and stats.get("n_m2l_kernel", 0) > 0 and stats["ms_m2l_kernel"] > 0:
@@ -679,13 +642,16 @@ def roofline(cfg, stats, peaks, fp64_tflops, fp32_tflops, tf32_tflops, phase=Non
     if dom == "m2l":
         Nd = stats.get("order_N") or cfg["N"]
         flops = float(m2l_flops(Nd)) * stats["n_far_pairs"]
-        R = Nd * (Nd + 1)
-        executed = 2.0 * R * R * stats["n_far_pairs"]
         achieved = flops / (ms * 1e-3) / 1e12
-        return {"kernel": "m2l_gemm_kernel (direction-grouped GEMM)", "bound": "fp64" if fp64 else "fp32",
-                "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-                "peak_source": src, "algorithmic_flops": flops, "executed_dense_flops": executed,
-                "executed_tflops": executed / (ms * 1e-3) / 1e12, "phase_ms": ms, "traffic": None}
+        # factored: six products of 8 x 4 FP64 MMA fragments per pair (a column
+        # of 64 flops each), without empty columns; SIMT FP32: the dense operator
+        frags = sum((n + 4) // 4 * ((n + 8) // 8) for n in range(Nd))
+        executed = (6 * 64.0 * frags if fp64 else 2.0 * (Nd * (Nd + 1)) ** 2) * stats["n_far_pairs"]
+        return {"kernel": "rot_kernel (factored FP64 M2L)" if fp64 else "m2l_gemm_kernel (SIMT FP32)",
+                "bound": "fp64" if fp64 else "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+                "frac": achieved / peak, "peak_source": src, "algorithmic_flops": flops,
+                "executed_flops": executed, "executed_tflops": executed / (ms * 1e-3) / 1e12, "phase_ms": ms,
+                "traffic": None}
     # tree / upward: HBM-bound passes over the particles
     nbytes = stats["n_particles"] * (2 * 32 + 2 * 8 + 4)
     achieved = nbytes / (ms * 1e-3) / 1e9
@@ -878,13 +844,6 @@ def run_batch(args, cfg):
     return 0
 
 
-def vector_launches(depth, precision):
-    """One tree, three scalar passes, the nonzero-charge, three component and
-    one cross-product kernels."""
-    tree, fmm = launches_per_solve(depth, 3, (3 * (depth - 1) + 7) // 8, True, precision, parts=True)
-    return tree + 3 * fmm + 1 + 3 + 1
-
-
 def run_vector(args, cfg):
     """Vector charges: the solve on device buffers, end to end through the
     host entry point, accuracy at 4096 targets against the FP64 direct sum
@@ -987,7 +946,7 @@ def run_vector(args, cfg):
                     "h2d_bytes_per_step": int(hs.numel() * 8 + hq.numel() * 8), "d2h_bytes_per_step": int(hf.numel() * 8)},
             "plain_fp64": {"value": n / (pms * 1e-3) / 1e6, "unit": "Mparticles/s", "ms_per_step": pms},
             "speedup_vs_plain_fp64": pms / ms, "cpu_baseline": cpu, "clocks": clk.summary(),
-            "gpu_launches": args.steps * vector_launches(depth, cfg["precision"])}
+            "gpu_launches": args.steps * traced_launches(torch, lambda: solve(cfg["precision"]))}
     ctx.close()
     print(json.dumps(line))
     return 0
@@ -1305,7 +1264,6 @@ def main():
         fp32 = fp32_peak_tflops(torch)
         tf32 = tf32_peak_tflops(torch)
         stats = r["stats"]
-        radix_passes = (cfg["dim"] * (cfg["depth"] - 1) + 7) // 8
         line = {
             "metric": cfg.get("metric", METRIC), "value": aggregate_rate(cfg["n"], world, r["ms"]), "unit": "Mparticles/s",
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": r["ms"],
@@ -1320,9 +1278,7 @@ def main():
             "roofline_leaves": roofline(cfg, stats, peaks, fp64, fp32, tf32, phase="leaves"),
             "fp64_peak_tflops_measured": fp64, "fp32_peak_tflops_measured": fp32, "tf32_peak_tflops_measured": tf32,
             "peaks_source": peaks["source"], "e2e": r["e2e"], "clocks": r["clocks"],
-            "gpu_launches": args.steps * launches_per_solve(stats["depth"], cfg["dim"], radix_passes,
-                                                            cfg.get("max_leaf", 0) > 0, cfg["precision"],
-                                                            learned=bool(r["learned"])),
+            "gpu_launches": args.steps * r["launches"],
         }
         if r["learned"]:
             line["learned_order"] = dict(r["learned"], tol=cfg["tol"], check_targets=cfg["check_targets"])
