@@ -101,19 +101,30 @@ __device__ __forceinline__ double quotient_refined(double q, double x, bool plai
 	return fma(fma(-p, x, q), y, p);
 }
 
-// Spherical coordinates with the reference's conventions
-// (common/simple_math.h:101-117): r gets +1e-12, phi = 0 on the z-axis,
-// +-pi/2 when |x| < 1e-12.
-template <typename real>
-__device__ __forceinline__ void dec_to_sph(real x, real y, real z, real& r, real& th, real& ph)
+// FP64 tensor-core MMA (mma.sync m8n8k4): D = A B + D, A 8x4 (lane: row lane/4,
+// column lane%4), B 4x8 (lane: row lane%4, column lane/4), D 8x8 (lane: row
+// lane/4, columns 2 (lane%4) + 0, 1).
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b)
 {
-	const real e = real(1e-12);
-	r = sqrt(x * x + y * y + z * z) + e;
-	th = acos(z / r);
-	if (fabs(x) + fabs(y) < e) ph = real(0);
-	else if (fabs(x) < e) ph = y / fabs(y) * real(PI * 0.5);
-	else ph = atan2(y, x);
+	asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+	             : "+d"(d[0]), "+d"(d[1])
+	             : "d"(a), "d"(b));
 }
+
+// Asynchronous copies to shared memory: bytes < 16 fills the rest with zeros.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes = 16)
+{
+	const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* dst, const void* src)
+{
+	const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+	asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(PENDING) : "memory"); }
 
 // Morton helpers: spread / gather every dim-th bit.
 __host__ __device__ inline uint64_t spread3(uint64_t v)

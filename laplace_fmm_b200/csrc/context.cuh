@@ -51,8 +51,7 @@ struct DevTables {
 	// per integer direction (dx+3)*49+(dy+3)*7+(dz+3):
 	// {dslot(theta), dslot(-theta), eslot(phi), eslot(-phi)}, -1 if absent
 	int4* dirinfo = nullptr;
-	// K(n,m) and the translation coefficient cubes [j][k][n] (18^3)
-	double* knm = nullptr;
+	// translation coefficient cubes [j][k][n] (18^3)
 	double* m2l = nullptr;
 	double* m2m = nullptr;
 	double* l2l = nullptr;
@@ -65,8 +64,9 @@ struct Tables {
 	std::vector<int4> dirinfo_host;
 };
 
-// Dense M2L operators [343][MT][MT] of one (order, cell size, precision),
-// kept across solves (repeated solves of one geometry rebuild nothing).
+// Operators or tables of one (order, cell size, kind), kept across solves: the
+// mixed form's M2L and M2M operators, the low orders' FP64 M2L operators, the 2D
+// M2L's.
 struct OpCacheEntry {
 	int N = 0, prec = 0;
 	double h = 0.0;
@@ -85,7 +85,9 @@ struct Context {
 	Tables tables;
 	std::vector<OpCacheEntry> opcache;
 	unsigned long long opcache_clock = 0;
-	int m2l_engine = 3;               // 0: dense SIMT GEMMs, 1: per-pair rotations (plain path), 3: tcgen05 on FP32 levels
+	// LFMM_M2L, 3D: 3 (tc, the default) or 0 (simt): tcgen05 or SIMT GEMMs on the mixed form's FP32 levels;
+	// 1 (rotation): per-pair rotations on the plain path.  2D: 1 per-pair, 0 dense GEMMs, 3 the Hankel form.
+	int m2l_engine = 3;
 	unsigned* dev_flags = nullptr;      // device error flags
 	// Device errors of asynchronous solves (device buffers, no stats): latched
 	// at the end of each such solve into this mapped pinned word (host view,
@@ -114,8 +116,7 @@ struct Context {
 	int timing = 0;
 };
 
-// With 48 entries cached (four per order: FP64 and tensor-core M2L, M2M and
-// L2L operators), evict the least recently used one no graph reads.
+// With 48 entries cached, evict the least recently used one no graph reads.
 inline void opcache_make_room(Context& ctx)
 {
 	if (ctx.opcache.size() < 48) return;

@@ -321,26 +321,15 @@ __device__ __forceinline__ void p2l_sum(const DevTree& t, size_t g, uint32_t xb,
 			const int32_t C = t.x_idx[e0 + lane];
 			b = t.pbeg[C]; n = t.send[C] - b;
 		}
-		uint32_t pre = n;                      // inclusive prefix sums of the entries' sources
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			const uint32_t v = __shfl_up_sync(0xffffffffu, pre, o);
-			if (lane >= o) pre += v;
-		}
-		const uint32_t total = __shfl_sync(0xffffffffu, pre, 31), first = b - (pre - n);
-		for (uint32_t f0 = 32u * w; f0 < total; f0 += 32u * nw) {
-			const uint32_t f = f0 + lane;
-			int k = 0;                         // the entry of source f: the prefixes <= f
-#pragma unroll
-			for (int o = 16; o > 0; o >>= 1)
-				if (__shfl_sync(0xffffffffu, pre, k + o - 1) <= f) k += o;
-			const uint32_t i = f + __shfl_sync(0xffffffffu, first, k & 31);
+		const SourceRun run(b, n);
+		for (uint32_t f0 = 32u * w; f0 < run.total; f0 += 32u * nw) {
+			const uint32_t f = f0 + lane, i = run.at(f);
 			real q = 0, x = 0, y = 0, z = 1;   // past the end: q = 0 at a finite point
-			if (f < total) {
+			if (f < run.total) {
 				q = (real)t.q[i];
 				x = (real)((t.x[i] - cx) * ih); y = (real)((t.y[i] - cy) * ih); z = (real)((t.z[i] - cz) * ih);
 			}
-			chain_add32<true, real, STEPS>(A, tb, q, x, y, z, (int)min(32u, total - f0), N);
+			chain_add32<true, real, STEPS>(A, tb, q, x, y, z, (int)min(32u, run.total - f0), N);
 		}
 	}
 }

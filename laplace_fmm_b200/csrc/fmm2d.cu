@@ -464,29 +464,18 @@ __global__ void __launch_bounds__(WPB2 * 32) p2l2d_kernel(DevTree t, Exp2 E)
 			const int32_t C = t.x_idx[e0 + lane];
 			b = t.pbeg[C]; n = t.send[C] - b;
 		}
-		uint32_t pre = n;                      // inclusive prefix sums of the entries' sources
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			const uint32_t v = __shfl_up_sync(0xffffffffu, pre, o);
-			if (lane >= o) pre += v;
-		}
-		const uint32_t total = __shfl_sync(0xffffffffu, pre, 31), first = b - (pre - n);
-		for (uint32_t f0 = 0; f0 < total; f0 += 32) {
-			const uint32_t f = f0 + lane;
-			int k = 0;                         // the entry of source f: the prefixes <= f
-#pragma unroll
-			for (int o = 16; o > 0; o >>= 1)
-				if (__shfl_sync(0xffffffffu, pre, k + o - 1) <= f) k += o;
-			const uint32_t i = f + __shfl_sync(0xffffffffu, first, k & 31);
+		const SourceRun run(b, n);
+		for (uint32_t f0 = 0; f0 < run.total; f0 += 32) {
+			const uint32_t f = f0 + lane, i = run.at(f);
 			double q = 0.0;
 			double2 z = make_double2(0.0, 0.0);
-			if (f < total) {
+			if (f < run.total) {
 				q = t.q[i];
 				const double dx = t.x[i] - cx, dy = t.y[i] - cy, r2 = dx * dx + dy * dy;
 				z = make_double2(dx / r2, -dy / r2);
 				lg.x += q * 0.5 * log(r2); lg.y -= q * atan2(-dy, -dx);
 			}
-			P.add32(z, q, (int)min(32u, total - f0), N);
+			P.add32(z, q, (int)min(32u, run.total - f0), N);
 		}
 	}
 	P.reduce();

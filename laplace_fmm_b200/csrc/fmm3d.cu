@@ -278,15 +278,6 @@ __global__ void __launch_bounds__(WPB * 32) m2l_ops_kernel(int N, int MT, double
 	}
 }
 
-
-// The plain form's kernels need no constant tables (the (n, m) of a
-// triangular index is computed: tri_row); kept as the solvers' setup hook.
-int upload_constants(Context& ctx)
-{
-	(void)ctx;
-	return OK;
-}
-
 } // namespace
 
 int m2l_ops_build(Context& ctx, int N, double h, double* out)
@@ -313,11 +304,10 @@ double* m2l_ops_fp64(Context& ctx, int N, double h)
 }
 
 int fmm3d_solve_device(Context& ctx, const ParticleInput& in, int N, int depth, double* pot, double* field,
-                       SolveStats* stats, DevTree* tree_out, double2** inner_out, double2** outer_out)
+                       SolveStats* stats, DevTree* tree_out)
 {
 	if (N < 1 || N > MAXN3) { ctx.last_error = "order out of range (1 <= N <= 18)"; return ERR_ARG; }
-	int st = upload_constants(ctx);
-	if (st) return st;
+	int st;
 	cudaStream_t s = ctx.stream;
 	const bool timing = ctx.timing != 0;
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[0], s));
@@ -414,8 +404,6 @@ int fmm3d_solve_device(Context& ctx, const ParticleInput& in, int N, int depth, 
 		}
 	}
 	if (tree_out) *tree_out = t;
-	if (inner_out) *inner_out = E.inner;
-	if (outer_out) *outer_out = E.outer;
 	return OK;
 }
 

@@ -18,8 +18,7 @@ struct SolveStats {
 // device pointers, n_out = nt if nt > 0 else ns.  N = number of degrees
 // (order p + 1), depth = uniform tree depth (levels), both already resolved.
 int fmm3d_solve_device(Context& ctx, const ParticleInput& in, int N, int depth, double* pot, double* field,
-                       SolveStats* stats, DevTree* tree_out = nullptr, double2** inner_out = nullptr,
-                       double2** outer_out = nullptr);
+                       SolveStats* stats, DevTree* tree_out = nullptr);
 
 // Scaled-expansion solver on the adaptive-form tree (max_leaf = 0: uniform
 // depth `depth`; > 0: adaptive, at most `depth` levels): precision 0 = FP64,

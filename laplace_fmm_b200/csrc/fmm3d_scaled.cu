@@ -213,7 +213,7 @@ int solve_t(Context& ctx, const DevTree& t, int N, double* pot, double* field, S
 	using v2 = typename V2<real>::t;
 	cudaStream_t s = ctx.stream;
 	const bool timing = ctx.timing != 0;
-	const int Nx2 = N * (N + 1) / 2, R = 2 * Nx2;
+	const int Nx2 = N * (N + 1) / 2;
 	const size_t C = t.ncells;
 	v2* outer = static_cast<v2*>(ctx.arena.take(sizeof(v2) * C * Nx2));
 	v2* inner = static_cast<v2*>(ctx.arena.take(sizeof(v2) * C * Nx2));
@@ -462,7 +462,6 @@ int fmm3d_scaled_on_tree(Context& ctx, const DevTree& t, int N, int precision, d
 	}
 	int st = upload_scaled_constants(ctx);
 	if (st) return st;
-	cudaStream_t s = ctx.stream;
 	const bool timing = ctx.timing != 0;
 	st = precision == 1 ? solve_t<float>(ctx, t, N, pot, field, stats, level_N)
 	                    : solve_t<double>(ctx, t, N, pot, field, stats, level_N);

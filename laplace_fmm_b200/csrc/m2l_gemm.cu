@@ -238,25 +238,6 @@ __global__ void m2l2d_tab_kernel(int N, double h, double2* __restrict__ tab)
 	tab[e] = make_double2(f * px, f * py);
 }
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes)
-{
-	const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int PENDING>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(PENDING) : "memory"); }
-
-// FP64 tensor-core MMA (mma.sync m8n8k4, the FP64 path of sm_100): D = A B + C
-// with A 8x4 row-major (lane: A[lane/4][lane%4]), B 4x8 column-major
-// (lane: B[lane%4][lane/4]) and C, D 8x8 (lane: C[lane/4][2 (lane%4) + 0, 1]).
-__device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b)
-{
-	asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-	             : "+d"(d0), "+d"(d1)
-	             : "d"(a), "d"(b));
-}
-
 constexpr int H2_LD = 136;             // row stride (doubles) of the staged W: conflict-free B fragments
 
 // Dynamic shared memory of the Hankel kernel for order N (bytes).
@@ -378,7 +359,7 @@ __global__ void __launch_bounds__(128, MTL < 4 ? 4 : 3) m2l2d_hankel_kernel(cons
 			for (int mt = 0; mt < MTL; ++mt) {
 				const double af = sH[8 * mt + g + k0 + t4];
 #pragma unroll
-				for (int nt = 0; nt < 4; ++nt) dmma_8x8x4(sacc[mt][nt][0], sacc[mt][nt][1], af, bf[nt]);
+				for (int nt = 0; nt < 4; ++nt) dmma(sacc[mt][nt], af, bf[nt]);
 			}
 		}
 #pragma unroll
@@ -642,7 +623,7 @@ __global__ void __launch_bounds__(256, 1) m2l_gemm_dmma_kernel(const double* __r
 				if (mt < MTT) {
 					const double af = a_[(8 * mt + g) * DG_LD + 4 * ks + t4];
 #pragma unroll
-					for (int n = 0; n < 4; ++n) dmma_8x8x4(acc[i][n][0], acc[i][n][1], af, bf[n]);
+					for (int n = 0; n < 4; ++n) dmma(acc[i][n], af, bf[n]);
 				}
 			}
 		}

@@ -2,7 +2,7 @@
 // targets of one octant class and a share of its far slots); D[128 targets][NC
 // coefficients] in TMEM.  Operands are hi / lo pairs: FP16 for the M2L (the
 // default; operators and each level's multipoles scaled by exact powers of
-// two), TF32 for the M2M / L2L shifts and the LFMM_M2L_TYPE=tf32 M2L.  Warp roles:
+// two), TF32 for M2M and the LFMM_M2L_TYPE=tf32 M2L.  Warp roles:
 //   warps 0-3  producers, one target row per thread.  FP16 with TMA (the
 //              default M2L): the sources are split once per level into staged
 //              FP16 hi / lo rows (stage_f16_kernel); per K block lanes 0-7 of

@@ -69,26 +69,6 @@ __global__ void rot_axial_kernel(int N, RotSizes sz, bool scaled, DevTables T, d
 	out[((size_t)lv * ROT_AX + e) * F * 32 + i] = v;
 }
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src)
-{
-	const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* dst, const void* src)
-{
-	const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-	asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-
-// D = A B + D, A 8x4 (lane: row lane/4, column lane%4), B 4x8 (lane: row
-// lane%4, column lane/4), D 8x8 (lane: row lane/4, columns 2 (lane%4) + 0, 1)
-__device__ __forceinline__ void dmma(double (&d)[2], double a, double b)
-{
-	asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-	             : "+d"(d[0]), "+d"(d[1])
-	             : "d"(a), "d"(b));
-}
-
 template <typename real> struct C2;
 template <> struct C2<double> { using t = double2; };
 template <> struct C2<float> { using t = float2; };
@@ -280,7 +260,7 @@ __global__ void __launch_bounds__(RW * 32, RW == 8 ? 2 : 1) rot_kernel(const typ
 				}
 			}
 		}
-		asm volatile("cp.async.commit_group;\n" ::: "memory");
+		cp_async_commit();
 	};
 	auto load_rot = [&](double2 (&a)[KT], int slot_d, int q) {
 		const double2* f = rotf + ((size_t)slot_d * rot_frag0(MAXN3) + jf[q]) * 32 + lane;
@@ -346,7 +326,7 @@ __global__ void __launch_bounds__(RW * 32, RW == 8 ? 2 : 1) rot_kernel(const typ
 		const int p = __popc(mk), nct = (p + 7) >> 3;
 		const bool more = j + 1 < nl;
 		const double* ax = axial + (size_t)s_ax[sl] * F * 32;
-		asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+		cp_async_wait<0>();
 		__syncthreads();
 		{
 			// raw columns times e^{i m phi} -> planes; warp: 8 columns x 4 coefficients at a time

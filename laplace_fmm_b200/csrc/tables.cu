@@ -153,15 +153,8 @@ int tables_build(Context& ctx)
 				TH.dirinfo_host[id] = make_int4(find(dslot, (int)(th * 100)), find(dslot, (int)(-th * 100)),
 				                               find(eslot, (int)(ph * 100)), find(eslot, (int)(-ph * 100)));
 			}
-	// normalisation constants, reference special_functions.h:56-116 recurrences
-	std::vector<double> K(MAXN3 * (MAXN3 + 1) / 2), A(2 * MAXN3 * (2 * MAXN3 + 1) / 2);
-	K[0] = 1.0;
-	for (int n = 1; n < MAXN3; ++n) {
-		for (int m = 0; m <= n - 1; ++m) K[tix(n, m)] = K[tix(n - 1, m)] * (n - m) / (n + m);
-		K[tix(n, n)] = K[tix(n, n - 1)] / (2 * n);
-	}
-	for (int n = 1; n < MAXN3; ++n)
-		for (int m = 0; m <= n; ++m) K[tix(n, m)] = std::sqrt(K[tix(n, m)]);
+	// reference special_functions.h:56-116 recurrences
+	std::vector<double> A(2 * MAXN3 * (2 * MAXN3 + 1) / 2);
 	A[0] = 1.0;
 	for (int n = 1; n < 2 * MAXN3; ++n) {
 		for (int m = 0; m <= n - 1; ++m) A[tix(n, m)] = A[tix(n - 1, m)] * (n - m) * (n + m);
@@ -184,7 +177,6 @@ int tables_build(Context& ctx)
 	LFMM_CUDA(ctx, cudaMalloc(&T.dmat, dbytes));
 	LFMM_CUDA(ctx, cudaMalloc(&T.emat, sizeof(double2) * MAXN3 * T.n_eslots));
 	LFMM_CUDA(ctx, cudaMalloc(&T.dirinfo, sizeof(int4) * 343));
-	LFMM_CUDA(ctx, cudaMalloc(&T.knm, sizeof(double) * K.size()));
 	LFMM_CUDA(ctx, cudaMalloc(&T.m2l, sizeof(double) * C));
 	LFMM_CUDA(ctx, cudaMalloc(&T.m2m, sizeof(double) * C));
 	LFMM_CUDA(ctx, cudaMalloc(&T.l2l, sizeof(double) * C));
@@ -195,7 +187,6 @@ int tables_build(Context& ctx)
 	LFMM_CUDA(ctx, cudaMemcpyAsync(d_th, TH.theta_of_slot.data(), sizeof(double) * T.n_dslots, cudaMemcpyHostToDevice, s));
 	LFMM_CUDA(ctx, cudaMemcpyAsync(d_ph, TH.phi_of_slot.data(), sizeof(double) * T.n_eslots, cudaMemcpyHostToDevice, s));
 	LFMM_CUDA(ctx, cudaMemcpyAsync(T.dirinfo, TH.dirinfo_host.data(), sizeof(int4) * 343, cudaMemcpyHostToDevice, s));
-	LFMM_CUDA(ctx, cudaMemcpyAsync(T.knm, K.data(), sizeof(double) * K.size(), cudaMemcpyHostToDevice, s));
 	LFMM_CUDA(ctx, cudaMemcpyAsync(T.m2l, m2l.data(), sizeof(double) * C, cudaMemcpyHostToDevice, s));
 	LFMM_CUDA(ctx, cudaMemcpyAsync(T.m2m, m2m.data(), sizeof(double) * C, cudaMemcpyHostToDevice, s));
 	LFMM_CUDA(ctx, cudaMemcpyAsync(T.l2l, l2l.data(), sizeof(double) * C, cudaMemcpyHostToDevice, s));
@@ -213,7 +204,7 @@ int tables_build(Context& ctx)
 void tables_free(Tables& TH)
 {
 	DevTables& T = TH.d;
-	cudaFree(T.dmat); cudaFree(T.rotf); cudaFree(T.emat); cudaFree(T.dirinfo); cudaFree(T.knm);
+	cudaFree(T.dmat); cudaFree(T.rotf); cudaFree(T.emat); cudaFree(T.dirinfo);
 	cudaFree(T.m2l); cudaFree(T.m2m); cudaFree(T.l2l);
 	TH = Tables();
 }

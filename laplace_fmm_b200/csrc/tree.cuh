@@ -74,6 +74,33 @@ __device__ __forceinline__ double cell_size(const DevTree& t, size_t g)
 	return scale / (double)(1ull << L);
 }
 
+// The sources of up to 32 list entries (lane: the first source b and their number
+// n of its entry) as one sequence; every lane of the warp takes part.
+struct SourceRun {
+	uint32_t pre, first, total;            // inclusive prefix sums, first source less the sources before it
+	__device__ __forceinline__ SourceRun(uint32_t b, uint32_t n) : pre(n)
+	{
+		const int lane = threadIdx.x & 31;
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1) {
+			const uint32_t v = __shfl_up_sync(0xffffffffu, pre, o);
+			if (lane >= o) pre += v;
+		}
+		total = __shfl_sync(0xffffffffu, pre, 31);
+		first = b - (pre - n);
+	}
+	// the particle of source f (f < total; else any value): its entry is the
+	// number of prefixes <= f
+	__device__ __forceinline__ uint32_t at(uint32_t f) const
+	{
+		int k = 0;
+#pragma unroll
+		for (int o = 16; o > 0; o >>= 1)
+			if (__shfl_sync(0xffffffffu, pre, k + o - 1) <= f) k += o;
+		return f + __shfl_sync(0xffffffffu, first, k & 31);
+	}
+};
+
 // partition: split each leaf into sources then q == 0 targets; lists: build
 // the close lists and far counts.
 int tree_build(Context& ctx, const ParticleInput& in, int depth, DevTree& t, bool partition = true,

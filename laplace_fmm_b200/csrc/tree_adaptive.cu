@@ -151,7 +151,6 @@ __global__ void source_ranges_kernel(DevTree a)
 	a.tend[g] = a.pend[g];
 }
 
-// U and W lists of one leaf (pass 0: count, pass 1: fill at the offsets).
 struct UWCount { uint32_t u = 0, w = 0; };
 
 // The U and W entries of leaf B (level L, coords me) under its colleague C, in
@@ -257,43 +256,12 @@ __global__ void uw_many_kernel(DevTree a, int pass, uint32_t* __restrict__ ucnt,
 	coords<DIM>(a.code[g], me);
 	uint32_t nu = 0, nw = 0;
 	const uint32_t ub = pass ? a.u_off[li] : 0, wb = pass ? a.w_off[li] : 0;
-	int32_t stack[STACK];
 	const int nc = a.close_cnt[g];
 	const int32_t* cl = a.close_idx + (size_t)g * a.close_stride;
-	const size_t off = a.loff[L];
 	for (int e = 0; e < nc; ++e) {
-		int32_t C = (int32_t)(off + cl[e]);
-		if (a.is_leaf[C]) {
-			if (pass) a.u_idx[ub + nu] = C;
-			nu++;
-			continue;
-		}
-		int sp = 0;
-		{
-			size_t cb = a.loff[L + 1];
-			for (uint32_t k = a.beg[C]; k < a.end[C]; ++k) stack[sp++] = (int32_t)(cb + k);
-		}
-		while (sp > 0) {
-			int32_t D = stack[--sp];
-			int ld = a.lev[D];
-			int d[3];
-			coords<DIM>(a.code[D], d);
-			if (touch<DIM>(L, me, ld, d)) {
-				if (a.is_leaf[D]) {
-					if (pass) a.u_idx[ub + nu] = D;
-					nu++;
-				} else {
-					size_t cb = a.loff[ld + 1];
-					for (uint32_t k = a.beg[D]; k < a.end[D]; ++k) {
-						if (sp < STACK) stack[sp++] = (int32_t)(cb + k);
-						else atomicOr(flags, DEV_ERR_LIST_OVERFLOW);
-					}
-				}
-			} else {
-				if (pass) a.w_idx[wb + nw] = D;
-				nw++;
-			}
-		}
+		const UWCount n = uw_walk<DIM>(a, L, me, (int32_t)(a.loff[L] + cl[e]), pass ? a.u_idx + ub + nu : nullptr,
+		                               pass ? a.w_idx + wb + nw : nullptr, flags);
+		nu += n.u; nw += n.w;
 	}
 	// coarser adjacent leaves: leaf colleagues of the ancestors that touch B
 	int32_t A = g;
