@@ -142,6 +142,10 @@ void tables_free(Tables& t);
 // made the first one's launch fail; the two calls also took about 1 us).
 cudaError_t smem_limit(int device, const void* kernel, size_t bytes, bool max_shared = false);
 
+// After cudaMemcpyToSymbol: from pageable memory it may return before the copy
+// has arrived, and the contexts' streams do not wait for the default stream.
+inline cudaError_t constants_ready() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 // set last_error from a CUDA error; returns ERR_CUDA
 int cuda_fail(Context& ctx, cudaError_t e, const char* where);
 

@@ -669,6 +669,7 @@ int upload_2d_constants(Context& ctx)
 	lt.ln2_hi = (double)(float)ln2;
 	lt.ln2_lo = (double)(ln2 - (long double)lt.ln2_hi);
 	LFMM_CUDA(ctx, cudaMemcpyToSymbol(c_logtab, &lt, sizeof(lt)));
+	LFMM_CUDA(ctx, constants_ready());
 	g_binom_ready[ctx.device] = true;
 	return OK;
 }

@@ -54,6 +54,7 @@ int upload_scaled_constants(Context& ctx)
 	LFMM_CUDA(ctx, cudaMemcpyToSymbol(g_grad_d, grad_d, sizeof(grad_d)));
 	LFMM_CUDA(ctx, cudaMemcpyToSymbol(g_S_f, S_f, sizeof(S_f)));
 	LFMM_CUDA(ctx, cudaMemcpyToSymbol(g_S_d, S_d, sizeof(S_d)));
+	LFMM_CUDA(ctx, constants_ready());
 	g_scaled_const_ready[ctx.device] = true;
 	return OK;
 }

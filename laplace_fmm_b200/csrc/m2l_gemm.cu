@@ -720,6 +720,7 @@ int upload_slots(Context& ctx)
 	fact[0] = 1.0;
 	for (int k = 1; k < 64; ++k) fact[k] = fact[k - 1] * k;
 	LFMM_CUDA(ctx, cudaMemcpyToSymbol(c_fact, fact, sizeof(fact)));
+	LFMM_CUDA(ctx, constants_ready());
 	g_slots_uploaded[ctx.device] = true;
 	return OK;
 }

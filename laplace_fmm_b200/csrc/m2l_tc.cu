@@ -1134,6 +1134,7 @@ int upload_slot_dirs(Context& ctx)
 	if (!g_uploaded[ctx.device]) {
 		const M2LSlots& S = m2l_slots();
 		LFMM_CUDA(ctx, cudaMemcpyToSymbol(c_tc_slot_dir, S.slot_dir, sizeof(S.slot_dir)));
+		LFMM_CUDA(ctx, constants_ready());
 		g_uploaded[ctx.device] = true;
 	}
 	return OK;
