@@ -69,11 +69,12 @@ __device__ __forceinline__ void reference_point(double& x, double& y, double z)
 // 1,920 sources are off FP64 by 0.95 to 1.005 times as much (geometric means by
 // order and degree).  FP32 takes two particles per lane group at once for the
 // latencies of the compensation.
-// Issue bound.  A lane-per-particle form that summed the lanes' values through
-// shared memory took 840 M instructions and 1150 us for the P2L of 1,048,576
-// clustered particles at N = 16 (95.7k X entries), and 279 M for their P2M.
-// Compensating every step, not only the first six, takes the P2M of 16.8M
-// particles at N = 17 from 2.54 to 3.14 ms and their P2L from 5.2 to 6.2.
+// Issue slots 60 % busy at 16 warps per SM, the rest the chains' own latencies.
+// A lane-per-particle form that summed the lanes' values through shared memory
+// took 840 M instructions and 1150 us for the P2L of 1,048,576 clustered
+// particles at N = 16 (95.7k X entries), and 279 M for their P2M (this form: 416
+// and 129 M).  Compensating every step, not only the first six, takes the P2M of
+// 16.8M particles at N = 17 from 2.54 to 3.14 ms and their P2L from 5.2 to 6.2.
 constexpr int CHL = 8;
 // steps of the busiest lane (N = 17: 20, N = 18: 23)
 __host__ __device__ constexpr int chain_steps(int N) { return N <= 15 ? N : N == 16 ? 17 : N == 17 ? 20 : 23; }
@@ -638,10 +639,11 @@ __device__ __forceinline__ void eval_pass(const EvalPass<K>& p, const DevTree& t
 // near field already in the outputs: one warp per leaf at a time (from a
 // counter), each expansion's coefficients derived once per pass of at most
 // eval_cap targets.  Leaves with more than FAR_SHORT W entries go to `longs`.
-// FP32: bound by the rows' shared-memory reads and the issue of about 16
-// instructions per coefficient and target.  Before (a target per lane, rows in
-// degree order, square roots in the derivation, one warp for a list of any
-// length) 300,007 clustered particles at N = 16 took 2640 us.
+// FP32: about 16 instructions per coefficient and target on rows read as 16-byte
+// broadcasts; 1,000,000 clustered particles at N = 16: 392 us, issue slots 52 %
+// busy, the largest stall the expansions' and targets' loads.  Before (a target
+// per lane, rows in degree order, square roots in the derivation, one warp for a
+// list of any length) 300,007 clustered particles at N = 16 took 2640 us.
 template <typename real>
 __global__ void __launch_bounds__(FWPB * 32, sizeof(real) == sizeof(float) ? 5 : 4) eval_scaled_kernel(DevTree t, const typename V2<real>::t* __restrict__ outer,
                                                                const typename V2<real>::t* __restrict__ inner, int N,

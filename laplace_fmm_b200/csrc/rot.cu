@@ -114,8 +114,8 @@ size_t rot_smem_limit(int N, size_t elem)
 // the columns present only.  The matrices' fragments come from L2 (25 KB per
 // slot at N = 9, 110 KB at N = 18), loaded for the next product before the
 // barrier that precedes it.
-// What bounds it: the FP64 MMAs are about a quarter of the time (N = 9: 26 %
-// of the tensor pipe), the rest is the four barriers and load latencies of a
+// What bounds it: the FP64 MMAs are about a third of the time (N = 9: 31 % of
+// the tensor pipe's active cycles), the rest is the four barriers and latencies of a
 // slot, which is why a warp holds at most two jobs and an SM 16 warps (with 8
 // warps of up to four jobs at N = 18 the M2L of 56k pairs took 491 us instead
 // of 279).  Against dense operators on the same pipe (m8n8k4 MMAs over the

@@ -143,7 +143,7 @@ def test_wigner_tables_match_oracle(ctx, oracle):
 
 @pytest.mark.parametrize("N,depth", [(9, 5), (13, 4), (6, 6)])
 def test_m2l_engines_agree(ctx, oracle, N, depth):
-    """Dense direction-GEMM M2L and per-pair rotations: both at parity."""
+    """Factored M2L (dense GEMMs at the low orders) and per-pair rotations: both at parity."""
     import os
     from laplace_fmm_b200 import Context
     os.environ["LFMM_M2L"] = "rotation"

@@ -1,9 +1,10 @@
-"""tcgen05 engine (hi/lo split, per-slot FP32 flush; the default for the
-mixed form's M2L, M2M and L2L: FP16 operands for the M2L, TF32 for the
-shifts) against the SIMT FP32 engine (SIMT GEMM M2L, rotation M2M / L2L), the
-TF32-operand M2L and the FP64 form.  The mixed engines must stay within the
-mixed form's 1e-6 of the FP64 form (measured: 3-5e-7 for the tensor-core
-engine; 1.1e-6 before L2L's diagonal moved out of the TF32 operators)."""
+"""tcgen05 engine (hi/lo split, per-slot FP32 flush; the mixed form's M2L on
+levels of more than 512 cells from level 4 on, FP16 operands) against the SIMT
+FP32 GEMM, the TF32-operand M2L and the FP64 form.  The mixed engines must stay
+within the mixed form's 1e-6 of the FP64 form (measured: 2-5e-7).  The other
+translations of these trees (M2M up to 6,144 cells, L2L, small levels) run
+factored in FP64; the tensor-core M2M of larger levels is in
+test_large_levels_gpu.py."""
 import os
 
 import pytest
@@ -96,10 +97,9 @@ def test_tc_engine_uniform(tc, simt, ctx, N):
 
 
 def test_tc_shifts_keep_fp32_accuracy(tc, ctx):
-    """M2M / L2L on the tensor cores (dense operators, L2L's diagonal applied
-    in FP32) stay as accurate as the rotation shifts: measured 3.6e-7 against
-    3.7e-7; with the diagonal left inside the TF32 operator this case measured
-    1.14e-6 (the dominant local coefficients lose 2^-22 at every level)."""
+    """Mixed solves whose M2M and L2L (factored, FP64 on FP32 expansions; dense
+    TF32 operators with L2L's diagonal in FP32 before, 3.6e-7, and 1.14e-6 with
+    the diagonal in TF32) stay within half of the mixed form's bar."""
     src, q = uniform3d(262144, seed=53)
     a = FastMultipole3d((src, q), N=13, tree_depth=6, precision="mixed", ctx=tc)
     c = FastMultipole3d((src, q), N=13, tree_depth=6, ctx=ctx)
