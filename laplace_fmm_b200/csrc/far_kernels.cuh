@@ -683,6 +683,7 @@ __global__ void __launch_bounds__(FWPB * 32, sizeof(real) == sizeof(float) ? 5 :
 			for (int j = 0; j < K; ++j)
 				if (p.g == 0 && p.idx(j) < np) {
 					const size_t r = t.orig[p.at(j)];
+					if (r >= t.n_out()) continue;
 					pot_out[r] += o[j][0];
 					fld_out[3 * r] += o[j][1]; fld_out[3 * r + 1] += o[j][2]; fld_out[3 * r + 2] += o[j][3];
 				}
@@ -754,7 +755,9 @@ __global__ void __launch_bounds__(FWL * 32, 2) eval_long_kernel(DevTree t, const
 				double v = 0.0;
 				for (int q = 0; q < FWL; ++q) v += part[q][tt][k];
 				const size_t r = t.orig[tb + k0 + tt];
-				if (k == 0) pot_out[r] += v; else fld_out[3 * r + k - 1] += v;
+				if (r < t.n_out()) {
+					if (k == 0) pot_out[r] += v; else fld_out[3 * r + k - 1] += v;
+				}
 			}
 		}
 	}
@@ -823,8 +826,10 @@ __global__ void __launch_bounds__(LW * 32) p2p_f64_kernel(DevTree t, double* __r
 			if (ti < np && ph == 0) {
 				if (!tmode) pot += t.q[i] * (1.0 / FORCE_EPS);
 				const size_t o = t.orig[i];
-				pot_out[o] = pot;
-				fld_out[3 * o] = fx; fld_out[3 * o + 1] = fy; fld_out[3 * o + 2] = fz;
+				if (o < t.n_out()) {
+					pot_out[o] = pot;
+					fld_out[3 * o] = fx; fld_out[3 * o + 1] = fy; fld_out[3 * o + 2] = fz;
+				}
 			}
 		}
 	}
@@ -955,7 +960,9 @@ __global__ void __launch_bounds__(FWL * 32, 2) leaves_plain_kernel(DevTree t, co
 			double v = 0.0;
 			for (int q = 0; q < FWL; ++q) v += part[q][tt][k];
 			const size_t r = t.orig[t0 + tt];
-			if (k == 0) pot_out[r] = v; else fld_out[3 * r + k - 1] = v;
+			if (r < t.n_out()) {
+				if (k == 0) pot_out[r] = v; else fld_out[3 * r + k - 1] = v;
+			}
 		}
 	}
 }

@@ -431,9 +431,11 @@ __global__ void __launch_bounds__(LW2 * 32) leaves2d_kernel(DevTree t, Exp2 E, c
 				}
 				pw = cmul(pw, dz);
 			}
-			const uint32_t o = t.orig[i];
-			pot_out[o] = pot;
-			fld_out[2 * (size_t)o] = fr; fld_out[2 * (size_t)o + 1] = fi;
+			const size_t o = t.orig[i];
+			if (o < t.n_out()) {
+				pot_out[o] = pot;
+				fld_out[2 * o] = fr; fld_out[2 * o + 1] = fi;
+			}
 		}
 	}
 }
@@ -634,9 +636,11 @@ __global__ void __launch_bounds__(LW2 * 32) leaves2d_adaptive_kernel(DevTree t, 
 			}
 			pw = cmul(pw, dz);
 		}
-		const uint32_t o = t.orig[i];
-		pot_out[o] = pot;
-		fld_out[2 * (size_t)o] = fr; fld_out[2 * (size_t)o + 1] = fi;
+		const size_t o = t.orig[i];
+		if (o < t.n_out()) {
+			pot_out[o] = pot;
+			fld_out[2 * o] = fr; fld_out[2 * o + 1] = fi;
+		}
 	}
 }
 
@@ -763,7 +767,7 @@ int fmm2d_solve_device(Context& ctx, const ParticleInput& in, int N, int depth, 
 		leaf_units_kernel<<<div_up(nl, 256), 256, 0, s>>>(t, units);
 		scan_exclusive_u32(units, units + nl, nl, units + 2 * nl, scr, s);
 		// at most one unit per leaf plus one per 32 targets
-		const size_t max_units = nl + (n_out + 31) / 32;
+		const size_t max_units = nl + (t.targets_num ? t.targets_num : t.n) / 32;   // of all leaves' targets
 		leaves2d_kernel<<<div_up(max_units, LW2), LW2 * 32, 0, s>>>(t, E, units + nl, units + 2 * nl, pot, field);
 	}
 	if (timing) LFMM_CUDA(ctx, cudaEventRecord(ctx.ev[5], s));
@@ -828,7 +832,7 @@ int fmm2d_solve_adaptive(Context& ctx, const ParticleInput& in, int N, int depth
 		if (!units || !scr) { ctx.last_error = "fmm2d: device allocation failed"; return ERR_OOM; }
 		leaf_units_adaptive_kernel<<<div_up(nl, 256), 256, 0, s>>>(t, units);
 		scan_exclusive_u32(units, units + nl, nl, units + 2 * nl, scr, s);
-		const size_t max_units = nl + (n_out + 31) / 32;
+		const size_t max_units = nl + (t.targets_num ? t.targets_num : t.n) / 32;   // of all leaves' targets
 		leaves2d_adaptive_kernel<<<div_up(max_units, LW2), LW2 * 32, 0, s>>>(t, E, units + nl, units + 2 * nl, pot,
 		                                                                        field);
 	}

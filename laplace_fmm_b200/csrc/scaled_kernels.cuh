@@ -274,9 +274,11 @@ __global__ void __launch_bounds__(LW * 32, 768 / (LW * 32)) p2p_f32_kernel(DevTr
 			}
 			if (valid && ph == 0) {
 				if (!tmode) pot += t.q[i] * (1.0 / FORCE_EPS);
-				const uint32_t o = t.orig[i];
-				pot_out[o] = pot;
-				fld_out[3 * (size_t)o] = fx; fld_out[3 * (size_t)o + 1] = fy; fld_out[3 * (size_t)o + 2] = fz;
+				const size_t o = t.orig[i];
+				if (o < t.n_out()) {
+					pot_out[o] = pot;
+					fld_out[3 * o] = fx; fld_out[3 * o + 1] = fy; fld_out[3 * o + 2] = fz;
+				}
 			}
 		}
 	}

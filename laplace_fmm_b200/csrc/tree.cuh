@@ -13,6 +13,10 @@ struct DevTree {
 	size_t n = 0;              // particles in the tree: [targets | sources]
 	size_t nt = 0;             // leading input particles that are targets (q = 0)
 	size_t targets_num = 0;    // particles with q == 0 (switches P2P to target mode)
+	// Outputs are written for the input particles below this: the targets given,
+	// or all particles.  With targets given, a source whose charge is zero lies
+	// among its leaf's targets but has no output.
+	__host__ __device__ size_t n_out() const { return nt ? nt : n; }
 	double* geo = nullptr;     // device: shift x, y, z, scale
 	double geo_host[4] = {};   // host copy
 	// particles in tree order (SoA)
