@@ -77,13 +77,16 @@ __device__ __forceinline__ bool beyond_1e300(double x) { return (unsigned)__doub
 // FP64 rounding for e < 2^-18, beside the roundings of x y (half of 2^-53) and of
 // the last sum (2^-53; measured 1.4e-16 in all).  The FP64 square root and divide
 // above 1e300.
-__device__ __forceinline__ double rsqrt_refined(double x)
+__device__ __forceinline__ double rsqrt_below_1e300(double x)
 {
-	if (beyond_1e300(x)) return 1.0 / sqrt(x);
 	double y;
 	asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
 	const double r = fma(-x * y, y, 1.0);
 	return fma(y * r, fma(r, 0.375, 0.5), y);
+}
+__device__ __forceinline__ double rsqrt_refined(double x)
+{
+	return beyond_1e300(x) ? 1.0 / sqrt(x) : rsqrt_below_1e300(x);
 }
 
 // q / x, x > 0; plain: |q| is below 1e300.  The hardware's FP64 reciprocal

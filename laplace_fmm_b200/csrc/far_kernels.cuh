@@ -766,8 +766,11 @@ __global__ void __launch_bounds__(FWL * 32, 2) eval_long_kernel(DevTree t, const
 // ---- near field of the FP64 form -------------------------------------------
 // One warp per leaf at a time (from a counter); targets in passes of up to 32,
 // fewer share the sources out between groups of lanes; sources of the leaf and
-// its U list staged 32 at a time.  Writes pot (with the reference's self term)
-// and field in input order; eval_scaled_kernel adds the expansions.
+// its U list staged 32 at a time, four of them per step of a lane, so that their
+// reciprocal square roots overlap (one at a time: 300,007 clustered particles 748
+// us, now 606; 8,475 in eight leaves, one warp each, 38 ms, now 15).  Writes pot
+// (with the reference's self term) and field in input order; eval_scaled_kernel
+// adds the expansions.
 template <int LW>
 __global__ void __launch_bounds__(LW * 32) p2p_f64_kernel(DevTree t, double* __restrict__ pot_out,
                                                          double* __restrict__ fld_out, unsigned* __restrict__ next_leaf)
@@ -805,16 +808,36 @@ __global__ void __launch_bounds__(LW * 32) p2p_f64_kernel(DevTree t, double* __r
 					}
 					__syncwarp();
 					const int self = sc_ == g ? (int)i - (int)s0 : -1;
-					for (int j = ph; j < cnt; j += G) {
-						const double4 s = ss[w][j];
-						const double dx = xi - s.x, dy = yi - s.y, dz = zi - s.z;
-						const double r2 = fmax(fma(dx, dx, fma(dy, dy, dz * dz)), FORCE_EPS2);
-						const double inv = rsqrt_refined(r2);
-						const double qi = j == self ? 0.0 : s.w * inv;
-						const double qi3 = qi * inv * inv;
-						pot += qi;
-						fx = fma(dx, qi3, fx); fy = fma(dy, qi3, fy); fz = fma(dz, qi3, fz);
-					}
+					auto pairs = [&](auto mc, int j) {
+						constexpr int M = decltype(mc)::value;
+						double dx[M], dy[M], dz[M], q[M], r2[M];
+						bool far = false;
+#pragma unroll
+						for (int m = 0; m < M; ++m) {
+							const double4 s = ss[w][j + m * G];
+							dx[m] = xi - s.x; dy[m] = yi - s.y; dz[m] = zi - s.z;
+							q[m] = j + m * G == self ? 0.0 : s.w;
+							r2[m] = fmax(fma(dx[m], dx[m], fma(dy[m], dy[m], dz[m] * dz[m])), FORCE_EPS2);
+							far |= beyond_1e300(r2[m]);
+						}
+						auto add = [&](int m, double inv) {
+							const double qi = q[m] * inv, qi3 = qi * inv * inv;
+							pot += qi;
+							fx = fma(dx[m], qi3, fx); fy = fma(dy[m], qi3, fy); fz = fma(dz[m], qi3, fz);
+						};
+						if (far) {
+							for (int m = 0; m < M; ++m) add(m, rsqrt_refined(r2[m]));
+						} else {
+							double inv[M];
+#pragma unroll
+							for (int m = 0; m < M; ++m) inv[m] = rsqrt_below_1e300(r2[m]);
+#pragma unroll
+							for (int m = 0; m < M; ++m) add(m, inv[m]);
+						}
+					};
+					int j = ph;
+					for (; j + 3 * G < cnt; j += 4 * G) pairs(std::integral_constant<int, 4>(), j);
+					for (; j < cnt; j += G) pairs(std::integral_constant<int, 1>(), j);
 				}
 			}
 			for (int o = 1 << lt; o < 32; o <<= 1) {
