@@ -74,7 +74,8 @@ __device__ __forceinline__ void reference_point(double& x, double& y, double z)
 // took 840 M instructions and 1150 us for the P2L of 1,048,576 clustered
 // particles at N = 16 (95.7k X entries), and 279 M for their P2M (this form: 416
 // and 129 M).  Compensating every step, not only the first six, takes the P2M of
-// 16.8M particles at N = 17 from 2.54 to 3.14 ms and their P2L from 5.2 to 6.2.
+// 16.8M particles at N = 17 from 2.54 to 2.66 ms and their P2L from 5.2 to 5.9
+// (P2M 3.14 with the totals of every step formed in every lane).
 constexpr int CHL = 8;
 // steps of the busiest lane (N = 17: 20, N = 18: 23)
 __host__ __device__ constexpr int chain_steps(int N) { return N <= 15 ? N : N == 16 ? 17 : N == 17 ? 20 : 23; }
@@ -238,32 +239,68 @@ __device__ __forceinline__ void chain_add32(ChainAcc<real, STEPS>& A, const Chai
 	for (; r < cnt; r += 4) chain_take<IRR, real, STEPS, 1>(A, tb, q, x, y, z, r, N);
 }
 
-// The four lane groups' sums added up (every lane ends with its steps'
-// totals); FP32: exact sums of two (Knuth), their errors carried in c.
-template <typename real, int STEPS>
-__device__ __forceinline__ void chain_reduce(ChainAcc<real, STEPS>& A, int N)
+// The four lane groups' sums added up: lane group u ends with the totals of the
+// steps 4 k + chain_sub() (a quarter of the exchanges of totals in every lane).
+// FP32: exact sums of two (Knuth), their errors carried in c, added in last.
+template <typename real> struct ChainVal {
+	typename V2<real>::t a, c;             // c: FP32 only
+};
+__device__ __forceinline__ int chain_sub() { return (threadIdx.x >> 3 & 1) | (threadIdx.x >> 3 & 2); }
+
+// keep the second (odd) or the first, plus the partner's (lane ^ o) of the same
+template <typename real>
+__device__ __forceinline__ ChainVal<real> chain_pair(const ChainVal<real>& x, const ChainVal<real>& y, bool odd, int o)
 {
-	const int T = chain_steps(N);
+	ChainVal<real> k = odd ? y : x;
+	const ChainVal<real> g = odd ? x : y;
+	typename V2<real>::t b;
+	b.x = __shfl_xor_sync(0xffffffffu, g.a.x, o);
+	b.y = __shfl_xor_sync(0xffffffffu, g.a.y, o);
+	if constexpr (sizeof(real) == sizeof(float)) {
+		const float2 d = make_float2(__shfl_xor_sync(0xffffffffu, g.c.x, o), __shfl_xor_sync(0xffffffffu, g.c.y, o));
+		const float2 a = k.a, u = add2(a, b), bv = sub2(u, a), err = add2(sub2(a, sub2(u, bv)), sub2(b, bv));
+		k.a = u;
+		k.c = add2(add2(k.c, d), err);
+	} else {
+		k.a.x += b.x; k.a.y += b.y;
+	}
+	return k;
+}
+
+template <typename real, int STEPS>
+__device__ __forceinline__ void chain_reduce(const ChainAcc<real, STEPS>& A, int N,
+                                             typename V2<real>::t (&tot)[(STEPS + 3) / 4])
+{
+	const int T = chain_steps(N), sub = chain_sub();
+	auto val = [&](int s) {
+		ChainVal<real> v;
+		v.a = s < STEPS ? A.a[s < STEPS ? s : 0] : V2<real>::make(0, 0);
+		if constexpr (sizeof(real) == sizeof(float)) v.c = s < STEPS ? A.c[s < STEPS ? s : 0] : make_float2(0.f, 0.f);
+		return v;
+	};
 #pragma unroll
-	for (int s = 0; s < STEPS; ++s) {
+	for (int k = 0; k < (STEPS + 3) / 4; ++k) {
+		if (4 * k >= T) break;
+		const ChainVal<real> lo = chain_pair<real>(val(4 * k), val(4 * k + 1), sub & 1, CHL);
+		const ChainVal<real> hi = chain_pair<real>(val(4 * k + 2), val(4 * k + 3), sub & 1, CHL);
+		const ChainVal<real> v = chain_pair<real>(lo, hi, sub & 2, 2 * CHL);
+		if constexpr (sizeof(real) == sizeof(float)) tot[k] = add2(v.a, v.c);
+		else tot[k] = v.a;
+	}
+}
+
+// out(index, total) for the coefficients whose totals this lane holds.
+template <typename real, int STEPS, typename F>
+__device__ __forceinline__ void chain_out(const ChainTab<real>& tb, int N, const typename V2<real>::t (&tot)[(STEPS + 3) / 4],
+                                          F out)
+{
+	const int T = chain_steps(N), l = threadIdx.x & (CHL - 1), sub = chain_sub();
+#pragma unroll
+	for (int k = 0; k < (STEPS + 3) / 4; ++k) {
+		const int s = 4 * k + sub;
 		if (s >= T) break;
-#pragma unroll
-		for (int o = CHL; o < 32; o <<= 1) {
-			typename V2<real>::t b;
-			b.x = __shfl_xor_sync(0xffffffffu, A.a[s].x, o);
-			b.y = __shfl_xor_sync(0xffffffffu, A.a[s].y, o);
-			if constexpr (sizeof(real) == sizeof(float)) {
-				const float2 a = A.a[s], u = add2(a, b);
-				A.a[s] = u;
-				const float2 d = make_float2(__shfl_xor_sync(0xffffffffu, A.c[s].x, o),
-				                             __shfl_xor_sync(0xffffffffu, A.c[s].y, o));
-				const float2 bv = sub2(u, a), err = add2(sub2(a, sub2(u, bv)), sub2(b, bv));
-				A.c[s] = add2(add2(A.c[s], d), err);
-			} else {
-				A.a[s].x += b.x; A.a[s].y += b.y;
-			}
-		}
-		if constexpr (sizeof(real) == sizeof(float)) A.a[s] = add2(A.a[s], A.c[s]);
+		const int o = tb.out[s * CHL + l];
+		if (o >= 0) out(o, tot[k]);
 	}
 }
 
@@ -278,8 +315,7 @@ __global__ void __launch_bounds__(FWPB * 32) p2m_scaled_kernel(DevTree t, int N,
 	__shared__ ChainTab<real> tb;
 	chain_tab_fill(tb, N, threadIdx.x, FWPB * 32);
 	__syncthreads();
-	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, l = lane % CHL;
-	const int Nx2 = N * (N + 1) / 2, T = chain_steps(N);
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, Nx2 = N * (N + 1) / 2;
 	for (size_t li = (size_t)blockIdx.x * FWPB + w; li < t.nleaves; li += (size_t)gridDim.x * FWPB) {
 		const size_t g = t.leaves[li];
 		const double ih = 1.0 / cell_size(t, g), cx = t.cx[g], cy = t.cy[g], cz = t.cz[g];
@@ -295,16 +331,10 @@ __global__ void __launch_bounds__(FWPB * 32) p2m_scaled_kernel(DevTree t, int N,
 			}
 			chain_add32<false, real, STEPS>(A, tb, q, x, y, z, (int)min(32u, e - base), N);
 		}
-		chain_reduce<real, STEPS>(A, N);
-		if (lane < CHL) {
-			typename V2<real>::t* out = outer + g * Nx2;
-#pragma unroll
-			for (int s = 0; s < STEPS; ++s) {
-				if (s >= T) break;
-				const int o = tb.out[s * CHL + l];
-				if (o >= 0) out[o] = V2<real>::make(A.a[s].x, -A.a[s].y);
-			}
-		}
+		typename V2<real>::t tot[(STEPS + 3) / 4];
+		chain_reduce<real, STEPS>(A, N, tot);
+		typename V2<real>::t* out = outer + g * Nx2;
+		chain_out<real, STEPS>(tb, N, tot, [&](int o, typename V2<real>::t v) { out[o] = V2<real>::make(v.x, -v.y); });
 	}
 }
 
@@ -359,8 +389,7 @@ __global__ void __launch_bounds__(FWPB * 32) p2l_kernel(DevTree t, int N, typena
 	__shared__ ChainTab<real> tb;
 	chain_tab_fill(tb, N, threadIdx.x, FWPB * 32);
 	__syncthreads();
-	const int lane = threadIdx.x & 31, l = lane % CHL;
-	const int Nx2 = N * (N + 1) / 2, T = chain_steps(N);
+	const int lane = threadIdx.x & 31, Nx2 = N * (N + 1) / 2;
 	const uint32_t cnt = shorts[0];
 	for (;;) {
 		uint32_t it = 0;
@@ -371,19 +400,13 @@ __global__ void __launch_bounds__(FWPB * 32) p2l_kernel(DevTree t, int N, typena
 		ChainAcc<real, STEPS> A;
 		A.clear();
 		p2l_sum<real, STEPS>(t, g, t.x_off[g], t.x_off[g + 1], 0, 1, N, tb, A);
-		chain_reduce<real, STEPS>(A, N);
-		if (lane < CHL) {
-			typename V2<real>::t* out = inner + g * Nx2;
-#pragma unroll
-			for (int s = 0; s < STEPS; ++s) {
-				if (s >= T) break;
-				const int o = tb.out[s * CHL + l];
-				if (o >= 0) {
-					const typename V2<real>::t a = out[o];
-					out[o] = V2<real>::make(a.x + A.a[s].x, a.y - A.a[s].y);
-				}
-			}
-		}
+		typename V2<real>::t tot[(STEPS + 3) / 4];
+		chain_reduce<real, STEPS>(A, N, tot);
+		typename V2<real>::t* out = inner + g * Nx2;
+		chain_out<real, STEPS>(tb, N, tot, [&](int o, typename V2<real>::t v) {
+			const typename V2<real>::t a = out[o];
+			out[o] = V2<real>::make(a.x + v.x, a.y - v.y);
+		});
 	}
 }
 
@@ -397,23 +420,16 @@ __global__ void __launch_bounds__(FWL * 32, sizeof(real) == sizeof(float) ? 2 : 
 	__shared__ typename V2<real>::t part[FWL][NX2MAX];
 	chain_tab_fill(tb, N, threadIdx.x, FWL * 32);
 	__syncthreads();
-	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, l = lane % CHL;
-	const int Nx2 = N * (N + 1) / 2, T = chain_steps(N);
+	const int w = threadIdx.x >> 5, Nx2 = N * (N + 1) / 2;
 	const uint32_t cnt = longs[0];
 	for (uint32_t it = blockIdx.x; it < cnt; it += gridDim.x) {
 		const size_t g = longs[1 + it];
 		ChainAcc<real, STEPS> A;
 		A.clear();
 		p2l_sum<real, STEPS>(t, g, t.x_off[g], t.x_off[g + 1], w, FWL, N, tb, A);
-		chain_reduce<real, STEPS>(A, N);
-		if (lane < CHL) {
-#pragma unroll
-			for (int s = 0; s < STEPS; ++s) {
-				if (s >= T) break;
-				const int o = tb.out[s * CHL + l];
-				if (o >= 0) part[w][o] = A.a[s];
-			}
-		}
+		typename V2<real>::t tot[(STEPS + 3) / 4];
+		chain_reduce<real, STEPS>(A, N, tot);
+		chain_out<real, STEPS>(tb, N, tot, [&](int o, typename V2<real>::t v) { part[w][o] = v; });
 		__syncthreads();
 		for (int c = threadIdx.x; c < Nx2; c += FWL * 32) {
 			double re = 0.0, im = 0.0;
@@ -869,8 +885,7 @@ __global__ void __launch_bounds__(FWPB * 32) p2m_plain_kernel(DevTree t, int N, 
 	__shared__ ChainTab<double> tb;
 	chain_tab_fill(tb, N, threadIdx.x, FWPB * 32);
 	__syncthreads();
-	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, l = lane % CHL, LL = t.depth - 1;
-	const int Nx2 = N * (N + 1) / 2, T = chain_steps(N);
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, LL = t.depth - 1, Nx2 = N * (N + 1) / 2;
 	const size_t leaf = (size_t)blockIdx.x * FWPB + w;
 	if (leaf >= t.lsize[LL]) return;
 	const size_t g = t.loff[LL] + leaf;
@@ -887,15 +902,9 @@ __global__ void __launch_bounds__(FWPB * 32) p2m_plain_kernel(DevTree t, int N, 
 		}
 		chain_add32<false, double, STEPS>(A, tb, q, x, y, z, (int)min(32u, e - base), N);
 	}
-	chain_reduce<double, STEPS>(A, N);
-	if (lane < CHL) {
-#pragma unroll
-		for (int s = 0; s < STEPS; ++s) {
-			if (s >= T) break;
-			const int o = tb.out[s * CHL + l];
-			if (o >= 0) outer[g * Nx2 + o] = make_double2(A.a[s].x, -A.a[s].y);
-		}
-	}
+	double2 tot[(STEPS + 3) / 4];
+	chain_reduce<double, STEPS>(A, N, tot);
+	chain_out<double, STEPS>(tb, N, tot, [&](int o, double2 v) { outer[g * Nx2 + o] = make_double2(v.x, -v.y); });
 }
 
 // Near field and (FAR) local expansion of 32 targets of a leaf on a block of
